@@ -7,11 +7,13 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 
 #include "gbspfft.h"
 #include "gbsp_internal.h"
 #include "gbsp_kernels.cuh"
+#include "gbsp_pass1_mma.cuh"
 
 // Returns a GBSP_ERR_* status (with the message recorded) from the calling
 // function when a CUDA runtime call fails.
@@ -52,6 +54,12 @@ int p1_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, const P
 int p1_batch_blocks_per_sm(const P1Kernel& k, size_t smem, int* nb);
 int p1_batch_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, const P1Args* args,
                     const long* item_begin, int nmat, unsigned long long* queue);
+
+// ---- pass 1 on the tensor cores (gbsp_pass1_mma.cu), one CTA per SM
+int p1_mma_prepare(size_t smem, bool batch);  // raises the limit, checks that it fits
+int p1_mma_launch(int sms, size_t smem, cudaStream_t st, const P1MmaArgs& a);
+int p1_mma_batch_launch(int grid, size_t smem, cudaStream_t st, const P1MmaArgs* args, const long* item_begin,
+                        int nmat, unsigned int* queue);
 
 // ---- Bluestein rows: mode ROW_*, compiled block bound ntmax (512 or 1024)
 struct RowsKernel {

@@ -41,6 +41,11 @@ struct gbsp_plan_s {
     int direct = 0;                  // one forward FFT of length cols per row (cols smooth), no Bluestein
     int* d_drev = nullptr;           // direct: where the forward network leaves each frequency
     int p1_ku = 8, p1_cw = 32;       // pass-1 rows per lane (x32 per item) and window width
+    int mma = 0;                     // pass 1 of large tiles on the tensor cores (k_twiddle_mma)
+    int mma_tab = 0, mma_ntab = 0;   // its twiddle table layout
+    size_t mma_smem = 0;
+    int* d_kptr = nullptr;           // mma: first K-step of every column
+    uint32_t* d_kfrac = nullptr;     // mma: row indices as fractions, padded to whole K-steps
     int p1_shape = 1;                // 1-based index of (p1_ku, p1_cw, tab_mode) in the shape table
     int planner = GBSP_PLANNER_MODEL;
     uint32_t rows_magic = 0;
@@ -208,6 +213,8 @@ gbsp::P1Kernel p1_kernel(const gbsp_plan_s* p) {
 
 // sizes pass 1's persistent grid (and raises the kernel's shared-memory limit)
 int p1_prepare(gbsp_plan_s* p, int sms) {
+    if (p->mma)
+        if (int rc = gbsp::p1_mma_prepare(p->mma_smem, false)) return rc;
     int nb = 0;
     if (int rc = gbsp::p1_blocks_per_sm(p1_kernel(p), p->p1_smem, &nb)) return rc;
     if (nb < 1) return set_error(GBSP_ERR_UNSUPPORTED, "pass-1 kernel does not fit on an SM");
@@ -239,13 +246,48 @@ gbsp::P1Args p1_args(const gbsp_plan_s* p, int u0, int n, float2* S, size_t s_pi
     return a;
 }
 
+gbsp::P1MmaArgs p1_mma_args(const gbsp_plan_s* p, int u0, int n, float2* S, size_t s_pitch, const float2* chirp) {
+    gbsp::P1MmaArgs a;
+    a.kfrac = p->d_kfrac;
+    a.kptr = p->d_kptr;
+    a.row_tab = p->d_rowtab;
+    a.chirp = chirp;
+    a.S = S;
+    a.s_pitch = s_pitch;
+    a.gtab = p->tab_mode;
+    a.tab = p->mma_tab;
+    a.ntab = p->mma_ntab;
+    a.cols = p->cols;
+    a.s_cols = p->s_cols;
+    a.rows = p->rows;
+    a.u0 = u0;
+    a.tile_rows = n;
+    gbsp::p1_mma_tiling(&a);
+    a.magic = p->rows_magic;
+    a.magic64 = p->rows_magic64;
+    a.queue = reinterpret_cast<unsigned int*>(p->d_err + 2);
+    a.err = p->d_err;
+    return a;
+}
+
 // The chirp pass 1 multiplies S by: the Bluestein pre-chirp (the channel-0
 // post table, chirp[c] * W^0), or none for direct plans.
 const float2* p1_chirp(const gbsp_plan_s* p) { return p->direct ? nullptr : p->d_post; }
 
+// The tensor-core kernel makes the operands of a nonzero at nearly the same
+// cost for any tile of up to 4096 rows, so it needs tall tiles, and enough
+// nonzeros per column to fill its K-steps.  Measured on GB300 (2048 columns,
+// uniform; FP32 time / tensor-core time at 1, 4, 12, 40, 120 nonzeros per
+// column): 1301 rows 0.84 0.97 0.97 1.05 1.15; 2051 rows 0.86 0.91 1.04 1.21
+// 1.38; 2751 rows 0.94 1.04 1.17 1.33 1.57; 6001 rows 1.13 1.25 1.44 1.71 1.92.
+constexpr int MMA_MIN_ROWS = 2048;
+constexpr long long MMA_MIN_ROWS_PER_COL = 10000;  // rows x nonzeros per column
+
 // chirp == nullptr gives the raw column sums (gbsp_column_sums)
 int launch_pass1(const gbsp_plan_s* p, int u0, int n, float2* S, size_t sp, const float2* chirp,
                  cudaStream_t st) {
+    if (p->mma && n >= MMA_MIN_ROWS)
+        return gbsp::p1_mma_launch(p->sms, p->mma_smem, st, p1_mma_args(p, u0, n, S, sp, chirp));
     return gbsp::p1_launch(p1_kernel(p), p->p1_grid, p->p1_smem, st, p1_args(p, u0, n, S, sp, chirp));
 }
 
@@ -359,6 +401,17 @@ int learned_choice(const gbsp_plan_s* p, const int* col_ptr, size_t smem_cap, gb
     return GBSP_OK;
 }
 
+// Whether the tensor-core kernel runs pass 1 of a plan's large tiles.  Not in
+// the exact-phase mode (no products of twiddles) nor with an explicit Kahan
+// degree (a property of the FP32 sums), nor with columns past its exact range.
+bool mma_choice(const gbsp_plan_s* p, const gbsp_options* o, const int* col_ptr) {
+    if (o->exact_phases != 0 || o->kahan_min_degree != 0 || p->mma_tab < 0) return false;
+    if (p->u_tile < MMA_MIN_ROWS || (long long)p->u_tile * p->nnz < MMA_MIN_ROWS_PER_COL * p->cols) return false;
+    int most = 0;
+    for (int j = 0; j < p->n_active; j++) most = std::max(most, col_ptr[j + 1] - col_ptr[j]);
+    return most <= gbsp::MM_MAX_DEGREE;
+}
+
 // force_p1: 1-based pass-1 shape imposed by a batch (one shape for all its
 // matrices); 0 leaves the choice to the options.
 int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int* sparse_cols,
@@ -434,6 +487,13 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
         p->ntab = (int)gbsp::row_table_entries(sh.tab, p->rows);
         p->p1_smem = gbsp::p1_smem_bytes(sh, p->rows);
     }
+    // the tensor-core kernel instead of that shape for large tiles
+    p->mma_tab = gbsp::mma_table(p->rows, smem_cap, p->tab_mode);
+    p->mma = mma_choice(p, &o, col_ptr);
+    if (p->mma) {
+        p->mma_ntab = (int)gbsp::row_table_entries(p->mma_tab, p->rows);
+        p->mma_smem = gbsp::p1_mma_smem_bytes(p->mma_ntab);
+    }
     if ((rc = p1_prepare(p, sms))) return rc;
 
     // ---- row-kernel configuration
@@ -449,6 +509,11 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
     const size_t off_task = (n_slot + 15) & ~(size_t)15;
     const size_t off_col = off_task + n_task * sizeof(int2);
     const size_t tbl_bytes = off_col + n_task;
+    // the K-step pointers (all columns | active columns) and indices of the
+    // tensor-core pass 1, built by k_kstep_scan and k_kstep_fill
+    const int n_kptr = (p->cols + gbsp::MM_MAXWIN - 1) / gbsp::MM_MAXWIN * gbsp::MM_MAXWIN + 1;
+    const size_t kptr_bytes = p->mma ? ((size_t)n_kptr + p->n_active + 1) * sizeof(int) : 0;
+    const size_t kfrac_bytes = p->mma ? ((size_t)p->nnz + 7 * (size_t)p->n_active + 8) * sizeof(uint32_t) : 0;
     // one device allocation for every buffer of the plan
     {
         // automatic streaming tile: ~half_rows / 9, to the nearest multiple
@@ -483,7 +548,8 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
                                 (p->row_mode == gbsp::ROW_SEQ || p->row_mode == gbsp::ROW_SEQW)
                                     ? (size_t)p->rows_grid * (K - 1) * Lp * sizeof(float2)
                                     : 0,
-                                stream_slab, stream_slab, p->direct ? (size_t)Lp * sizeof(int) : 0};
+                                stream_slab, stream_slab, p->direct ? (size_t)Lp * sizeof(int) : 0, kptr_bytes,
+                                kfrac_bytes};
         size_t total = 0;
         for (size_t b : sizes) total += a256(b);
         void* base = nullptr;
@@ -510,6 +576,9 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
     p->d_win_slot0 = d_tbl;
     p->d_win_task = reinterpret_cast<int2*>(d_tbl + off_task);
     p->d_win_task_col = d_tbl + off_col;
+    if (p->mma && ((rc = dev_alloc(p, (void**)&p->d_kptr, kptr_bytes)) ||
+                   (rc = dev_alloc(p, (void**)&p->d_kfrac, kfrac_bytes))))
+        return rc;
     if (stream_slab > 0) {
         for (int b = 0; b < 2; b++)
             if ((rc = dev_alloc(p, &p->stream_slab[b], stream_slab))) return rc;
@@ -610,6 +679,24 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
     if (e == cudaSuccess && na > 0)
         e = cudaMemcpyAsync(d_sc, sparse_cols, (size_t)na * sizeof(int), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && p->nnz > 0) e = cudaMemcpyAsync(d_in, row_idx, idx_in_bytes, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && p->mma) {
+        int* kact = p->d_kptr + n_kptr;
+        gbsp::k_kstep_scan<<<1, gbsp::KSCAN_THREADS, 0, st>>>(d_cp, na, kact);
+        gbsp::KstepFillArgs fa;
+        fa.col_ptr = d_cp;
+        fa.sparse_cols = d_sc;
+        fa.kact = kact;
+        fa.row_in = d_in;
+        fa.kptr = p->d_kptr;
+        fa.kfrac = p->d_kfrac;
+        fa.n_active = na;
+        fa.n_kptr = n_kptr;
+        fa.ptr_blocks = (int)blocks_for(n_kptr, gbsp::SETUP_WARPS * 32);
+        fa.rows = p->rows;
+        const int col_blocks = (int)std::min<long>(blocks_for(na, gbsp::SETUP_WARPS), (long)sms * 16);
+        gbsp::k_kstep_fill<<<fa.ptr_blocks + std::max(col_blocks, 1), gbsp::SETUP_WARPS * 32, 0, st>>>(fa);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess) {
         gbsp::CscSetupArgs ca;
         ca.col_ptr = d_cp;
@@ -901,6 +988,11 @@ struct gbsp_batch_s {
     int p1_shape = 1, ku = 8, cw = 32, tab = 0, idx_bytes = 2, big = 0, exact = 0;
     int p1_grid = 0;
     size_t p1_smem = 0;
+    // pass 1 of the matrices in `order`: FP32 (n_fp32) or tensor cores (n_mma)
+    int n_fp32 = 0, n_mma = 0, mma_grid = 0;
+    size_t mma_smem = 0;
+    gbsp::P1MmaArgs* d_mma = nullptr;
+    long* d_mma_begin = nullptr;
     // Row launches: one per class of matrices that share a block size and a
     // CTAs-per-SM count, so small rows keep the occupancy they have alone.
     struct RowsClass {
@@ -912,7 +1004,7 @@ struct gbsp_batch_s {
     long* d_p1_begin = nullptr;
     gbsp::RowsBatch* d_rows = nullptr;
     long* d_row_begin = nullptr;            // per class: count+1 prefix entries from 0
-    unsigned long long* d_queue = nullptr;  // [0] pass 1, [1 + c] rows of class c
+    unsigned long long* d_queue = nullptr;  // [0] pass 1, [1] its tensor-core part, [2 + c] rows of class c
     int* d_err = nullptr;
     std::vector<void*> outs;
     std::vector<size_t> pitches;
@@ -953,19 +1045,22 @@ int p1b_dispatch(gbsp_batch_s* b, bool prepare, int sms, cudaStream_t st) {
         b->p1_grid = nb * sms;
         return GBSP_OK;
     }
-    return gbsp::p1_batch_launch(k, b->p1_grid, b->p1_smem, st, b->d_p1, b->d_p1_begin, (int)b->order.size(),
-                                 b->d_queue);
+    return gbsp::p1_batch_launch(k, b->p1_grid, b->p1_smem, st, b->d_p1, b->d_p1_begin, b->n_fp32, b->d_queue);
 }
 
 int batch_launch(gbsp_batch_s* b, cudaStream_t st) {
     if (!b->order.empty()) {
-        GB_CUDA(cudaMemsetAsync(b->d_queue, 0, (1 + b->classes.size()) * sizeof(unsigned long long), st));
-        int rc = p1b_dispatch(b, false, 0, st);
-        if (rc) return rc;
+        GB_CUDA(cudaMemsetAsync(b->d_queue, 0, (2 + b->classes.size()) * sizeof(unsigned long long), st));
+        int rc = GBSP_OK;
+        if (b->n_mma > 0 &&
+            (rc = gbsp::p1_mma_batch_launch(b->mma_grid, b->mma_smem, st, b->d_mma, b->d_mma_begin, b->n_mma,
+                                            reinterpret_cast<unsigned int*>(b->d_queue + 1))))
+            return rc;
+        if (b->n_fp32 > 0 && (rc = p1b_dispatch(b, false, 0, st))) return rc;
         for (size_t c = 0; c < b->classes.size(); c++) {
             const auto& k = b->classes[c];
             if ((rc = gbsp::rows_batch_launch(k.grid, k.nt, k.smem, st, b->d_rows + k.begin,
-                                              b->d_row_begin + k.begin + c, k.end - k.begin, b->d_queue + 1 + c,
+                                              b->d_row_begin + k.begin + c, k.end - k.begin, b->d_queue + 2 + c,
                                               b->d_err)))
                 return rc;
         }
@@ -1093,35 +1188,52 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
     }
     const int ncls = (int)b->classes.size();
     if (n > 0) {
-        if ((rc = p1b_dispatch(b, true, sms, st)) ||
-            (rc = batch_alloc(b, (void**)&b->d_p1, sizeof(gbsp::P1Args) * n)) ||
-            (rc = batch_alloc(b, (void**)&b->d_p1_begin, sizeof(long) * (n + 1))) ||
+        // pass-1 lists in queue order, FP32 and tensor cores apart
+        std::vector<gbsp::P1Args> p1;
+        std::vector<gbsp::P1MmaArgs> mm;
+        std::vector<long> p1b(1, 0), mmb(1, 0), rb;
+        const int ublk = 32 * b->ku;
+        for (int k = 0; k < n; k++) {
+            const gbsp_plan_s* p = b->plans[b->order[k]];
+            if (p->mma) {
+                mm.push_back(p1_mma_args(p, 0, p->half_rows, p->d_S, p->s_pitch, p1_chirp(p)));
+                mmb.push_back(mmb.back() + gbsp::p1_mma_items(mm.back()));
+                b->mma_smem = std::max(b->mma_smem, p->mma_smem);
+                continue;
+            }
+            p1.push_back(p1_args(p, 0, p->half_rows, p->d_S, p->s_pitch, p1_chirp(p)));
+            p1b.push_back(p1b.back() +
+                          (long)((p->half_rows + ublk - 1) / ublk) * ((p->s_cols + p->p1_cw - 1) / p->p1_cw));
+        }
+        b->n_fp32 = (int)p1.size();
+        b->n_mma = (int)mm.size();
+        b->mma_grid = sms;
+        if ((b->n_fp32 > 0 && (rc = p1b_dispatch(b, true, sms, st))) ||
+            (b->n_mma > 0 && (rc = gbsp::p1_mma_prepare(b->mma_smem, true))) ||
+            (rc = batch_alloc(b, (void**)&b->d_p1, sizeof(gbsp::P1Args) * p1.size())) ||
+            (rc = batch_alloc(b, (void**)&b->d_p1_begin, sizeof(long) * p1b.size())) ||
+            (rc = batch_alloc(b, (void**)&b->d_mma, sizeof(gbsp::P1MmaArgs) * mm.size())) ||
+            (rc = batch_alloc(b, (void**)&b->d_mma_begin, sizeof(long) * mmb.size())) ||
             (rc = batch_alloc(b, (void**)&b->d_rows, sizeof(gbsp::RowsBatch) * n)) ||
             (rc = batch_alloc(b, (void**)&b->d_row_begin, sizeof(long) * (n + ncls)))) {
             free_batch(b);
             return rc;
         }
-        // work-queue prefix sums (pass 1 over the whole queue, rows per class)
-        std::vector<gbsp::P1Args> p1(n);
-        std::vector<long> p1b(n + 1, 0), rb;
-        const int ublk = 32 * b->ku;
-        for (int k = 0; k < n; k++) {
-            const gbsp_plan_s* p = b->plans[b->order[k]];
-            p1[k] = p1_args(p, 0, p->half_rows, p->d_S, p->s_pitch, p1_chirp(p));
-            p1b[k + 1] = p1b[k] + (long)((p->half_rows + ublk - 1) / ublk) * ((p->s_cols + p->p1_cw - 1) / p->p1_cw);
-        }
         for (const auto& c : b->classes) {
             rb.push_back(0);
             for (int k = c.begin; k < c.end; k++) rb.push_back(rb.back() + b->plans[b->order[k]]->half_rows);
         }
-        if (cudaMemcpy(b->d_p1, p1.data(), sizeof(gbsp::P1Args) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(b->d_p1_begin, p1b.data(), sizeof(long) * (n + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
+        if (cudaMemcpy(b->d_p1, p1.data(), sizeof(gbsp::P1Args) * p1.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaMemcpy(b->d_p1_begin, p1b.data(), sizeof(long) * p1b.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaMemcpy(b->d_mma, mm.data(), sizeof(gbsp::P1MmaArgs) * mm.size(), cudaMemcpyHostToDevice) !=
+                cudaSuccess ||
+            cudaMemcpy(b->d_mma_begin, mmb.data(), sizeof(long) * mmb.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
             cudaMemcpy(b->d_row_begin, rb.data(), sizeof(long) * rb.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
             free_batch(b);
             return set_error(GBSP_ERR_CUDA, "gbsp_batch_create: descriptor upload failed");
         }
     }
-    if ((rc = batch_alloc(b, (void**)&b->d_queue, (1 + ncls) * sizeof(unsigned long long))) ||
+    if ((rc = batch_alloc(b, (void**)&b->d_queue, (2 + ncls) * sizeof(unsigned long long))) ||
         (rc = batch_alloc(b, (void**)&b->d_err, sizeof(int)))) {
         free_batch(b);
         return rc;

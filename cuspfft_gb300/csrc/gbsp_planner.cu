@@ -254,6 +254,14 @@ std::vector<int> fitting_p1_shapes(int rows, size_t smem_cap, int table_mode) {
     return out;
 }
 
+int mma_table(int rows, size_t smem_cap, int plan_tab) {
+    for (int tab = plan_tab; tab <= TAB_TWO; tab++) {
+        if (tab != TAB_TWO && rows > 65535) continue;  // 64-bit phases: two-level only
+        if (p1_mma_smem_bytes(row_table_entries(tab, rows)) + 7168 <= smem_cap) return tab;  // + static variables
+    }
+    return -1;
+}
+
 int device_limits(int dev, DeviceLimits* out) {
     constexpr int kMaxDev = 64;
     static std::mutex mu;

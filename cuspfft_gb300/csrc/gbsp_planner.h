@@ -52,6 +52,11 @@ size_t p1_smem_bytes(const P1Shape& sh, int rows);
 // under the table mode (0 auto, 1 full, 2 half, 3 two-level).
 std::vector<int> fitting_p1_shapes(int rows, size_t smem_cap, int table_mode);
 
+// Table layout of the tensor-core pass 1 for `rows`: the first of full, half,
+// two-level that fits, no finer than the plan's own (`plan_tab`, which it is
+// made from); -1 when none fits.
+int mma_table(int rows, size_t smem_cap, int plan_tab);
+
 // Shared memory per CTA available to the kernels: the current device's
 // opt-in limit, or GB300's 232448 bytes when no device is visible.
 size_t device_smem_cap();

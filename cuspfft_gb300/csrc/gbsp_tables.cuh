@@ -135,6 +135,84 @@ __global__ void __launch_bounds__(SETUP_WARPS * 32) k_csc_setup(CscSetupArgs a) 
     }
 }
 
+// The CSC half of a plan's build for the tensor-core pass 1: every row index r
+// as ceil(r * 2^32 / rows), each column padded to whole K-steps of eight with
+// MM_PAD, and the first K-step of every column.
+//
+// k_kstep_scan (one block): kact[j], the first K-step of active column j, and
+// their total in kact[n_active].  A thread's contiguous share of the columns
+// is summed, the sums scanned over the block, the share written.
+// k_kstep_fill: blocks [0, ptr_blocks) write kptr[c] for n_kptr columns, one
+// thread each by a binary search in sparse_cols; the other blocks write one
+// active column per warp (row indices are checked by k_csc_setup).
+constexpr int KSCAN_THREADS = 1024;
+__global__ void __launch_bounds__(KSCAN_THREADS) k_kstep_scan(const int* __restrict__ col_ptr, int n_active,
+                                                              int* __restrict__ kact) {
+    __shared__ int wsum[KSCAN_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int per = (n_active + KSCAN_THREADS - 1) / KSCAN_THREADS;
+    const int j0 = min(tid * per, n_active), j1 = min(j0 + per, n_active);
+    int sum = 0;
+    for (int j = j0; j < j1; j++) sum += (col_ptr[j + 1] - col_ptr[j] + 7) >> 3;
+    int incl = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) wsum[tid >> 5] = incl;
+    __syncthreads();
+    if (tid < 32) {
+        int w = wsum[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += v;
+        }
+        wsum[lane] = w;
+    }
+    __syncthreads();
+    int at = incl - sum + (tid >= 32 ? wsum[(tid >> 5) - 1] : 0);
+    for (int j = j0; j < j1; j++) {
+        kact[j] = at;
+        at += (col_ptr[j + 1] - col_ptr[j] + 7) >> 3;
+    }
+    if (tid == KSCAN_THREADS - 1) kact[n_active] = at;
+}
+
+struct KstepFillArgs {
+    const int* col_ptr;
+    const int* sparse_cols;
+    const int* kact;
+    const int* row_in;
+    int* kptr;
+    uint32_t* kfrac;
+    int n_active, n_kptr, ptr_blocks, rows;
+};
+__global__ void __launch_bounds__(SETUP_WARPS * 32) k_kstep_fill(KstepFillArgs a) {
+    if ((int)blockIdx.x < a.ptr_blocks) {
+        const int c = blockIdx.x * blockDim.x + threadIdx.x;
+        if (c >= a.n_kptr) return;
+        int lo = 0, hi = a.n_active;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (a.sparse_cols[mid] < c) lo = mid + 1;
+            else hi = mid;
+        }
+        a.kptr[c] = a.kact[lo];
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    const int nw = (gridDim.x - a.ptr_blocks) * SETUP_WARPS;
+    for (int j = (blockIdx.x - a.ptr_blocks) * SETUP_WARPS + (threadIdx.x >> 5); j < a.n_active; j += nw) {
+        const int p0 = a.col_ptr[j], deg = a.col_ptr[j + 1] - p0;
+        const size_t at = (size_t)a.kact[j] * 8;
+        for (int i = lane; i < ((deg + 7) & ~7); i += 32) {
+            const uint32_t r = i < deg ? (uint32_t)a.row_in[p0 + i] : 0u;
+            a.kfrac[at + i] =
+                i < deg ? (uint32_t)((((unsigned long long)r << 32) + (uint32_t)a.rows - 1) / (uint32_t)a.rows) : MM_PAD;
+        }
+    }
+}
+
 // Chirp exp(-i*pi*c^2/cols) times W_L^{+c*q} (sign = +1) or W_L^{-c*q} (sign = -1),
 // W_L = exp(-2*pi*i/L); c^2 mod 2*cols and c*q mod L are reduced exactly.
 __device__ __forceinline__ float2 chirp_twiddle(long long c, int q, int cols, int L, int sign) {

@@ -63,7 +63,12 @@ enum { GBSP_PLANNER_MODEL = 0, GBSP_PLANNER_LEARNED = 1 };
  *   5: 256 x 16, half            6: 128 x 32, half
  *   7: 256 x 32, two-level       8: 128 x 32, two-level (tall matrices)
  * The automatic choice takes the first that fits of 1, 2, 7, 3, 4, 5, 6, 8
- * (measured on GB300); the tuner and the learned planner consider them all. */
+ * (measured on GB300); the tuner and the learned planner consider them all.
+ * Shapes are those of the FP32 pass 1.  Tiles of at least 2048 Bluestein rows
+ * of a matrix with at least 10000 / rows nonzeros per column and none above
+ * 1024 run pass 1 on the tensor cores instead, from the same table (sums
+ * closer to FP64 than the FP32 ones), unless exact_phases or kahan_min_degree
+ * is set. */
 #define GBSP_N_PASS1_SHAPES 8
 /* Length of the cost-model feature vector (gbsp_plan_features). */
 #define GBSP_N_FEATURES 36
@@ -81,7 +86,8 @@ typedef struct {
     int u_tile;            /* Bluestein rows per tile (each yields output rows u and
                               rows-u); the --csc-tile analogue. 0 = all rows in one tile */
     int kahan_min_degree;  /* columns with >= this many nonzeros accumulate with Kahan
-                              compensation; 0 = default 64; negative = never (plain FP32) */
+                              compensation; 0 = default 64; negative = never (plain FP32);
+                              any value but 0 keeps pass 1 on the FP32 kernel       */
     int index_bytes;       /* 0 = auto (2 when rows,cols <= 65536, else 4), or 2 / 4      */
     int max_channel_len;   /* largest per-CTA FFT length held in shared memory;
                               0 = as long as shared memory allows (about 28k points);
