@@ -520,6 +520,48 @@ struct RowsArgs {
     const int* drev;
 };
 
+// The fold of a row longer than its channel q: slot n gets
+// sum_j W_L^{q (n + j*Lp)} * x[n + j*Lp] over at most NS sections; with
+// W_L^{q (n + j*Lp)} = W_L^{q n} * W_K^{q j} (pre[n] and pre[j*Lp]) one table
+// entry per slot instead of one per value, and none for channel 0 (PRE false).
+// U slots a pass, all their loads (L2) issued before any product: one slot a
+// pass waited out the L2 latency Lp / nt times per channel, 46 % of the row
+// kernel on 40421 columns (three channels of 27000, two sections).
+template <bool PRE, int NS, int U>
+__device__ __forceinline__ void fold_sections(float2* __restrict__ buf, const float2* __restrict__ x,
+                                              const float2* __restrict__ pre, int cols, int Lp, int tid, int nt) {
+    float2 wk[NS];
+#pragma unroll
+    for (int j = 1; j < NS; j++) wk[j] = (PRE && j * Lp < cols) ? __ldg(pre + j * Lp) : make_float2(1.f, 0.f);
+    for (int n0 = tid; n0 < Lp; n0 += U * nt) {
+        float2 xv[U][NS], pv[U];
+#pragma unroll
+        for (int w = 0; w < U; w++) {
+            const int n = n0 + w * nt;
+#pragma unroll
+            for (int j = 0; j < NS; j++) {
+                const int c = n + j * Lp;
+                xv[w][j] = (n < Lp && c < cols) ? __ldcg(x + c) : make_float2(0.f, 0.f);
+            }
+            if (PRE) pv[w] = n < Lp ? __ldg(pre + n) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int w = 0; w < U; w++) {
+            float2 acc = xv[w][0];
+#pragma unroll
+            for (int j = 1; j < NS; j++) acc = cadd(acc, PRE ? cmul(xv[w][j], wk[j]) : xv[w][j]);
+            if (PRE) acc = cmul(acc, pv[w]);
+            if (n0 + w * nt < Lp) buf[n0 + w * nt] = acc;
+        }
+    }
+}
+template <int NS, int U>
+__device__ __forceinline__ void fold_channel(int q, float2* buf, const float2* x, const float2* pre, int cols, int Lp,
+                                             int tid, int nt) {
+    if (q == 0) fold_sections<false, NS, U>(buf, x, pre, cols, Lp, tid, nt);
+    else fold_sections<true, NS, U>(buf, x, pre, cols, Lp, tid, nt);
+}
+
 // How the K channels of a long row are laid out on the GPU.
 //   ROW_SINGLE  K == 1, one CTA per row
 //   ROW_CLUSTER one CTA per channel, the K CTAs of a row one thread-block
@@ -603,30 +645,17 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
             }
             __syncthreads();
         } else if constexpr (MULTI) {
-            // Several input columns fold onto one slot: slot n gets
-            // sum_j pre[n + j*Lp] * x[n + j*Lp].  Every channel reads the whole
-            // S row, so it is loaded to stay in L2 for the next channel (an
-            // evict-first load made each channel re-read it from DRAM).
-            // Each thread owns its slots, so
-            // no zero fill or barrier between sections; all of a slot's loads
-            // are issued before its products.
+            // Several input columns fold onto one slot.  Every channel reads
+            // the whole S row, so it is loaded to stay in L2 for the next
+            // channel (an evict-first load made each channel re-read it from
+            // DRAM).  Each thread owns its slots, so no zero fill or barrier
+            // between sections.
             // L = K*Lp >= 2*cols - 1 gives cols/Lp <= K/2 + 1/(2Lp): at most
             // K/2 + 1 sections
-            constexpr int MAXSEC = MAX_CHANNELS / 2 + 1;
-            for (int n = tid; n < Lp; n += nt) {
-                float2 xv[MAXSEC], pv[MAXSEC];
-#pragma unroll
-                for (int j = 0; j < MAXSEC; j++) {
-                    const int c = n + j * Lp;
-                    const bool ok = c < cols;
-                    xv[j] = ok ? __ldcg(srow + c) : make_float2(0.f, 0.f);
-                    pv[j] = ok ? __ldg(preq + c) : make_float2(0.f, 0.f);
-                }
-                float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int j = 0; j < MAXSEC; j++) acc = cadd(acc, cmul(xv[j], pv[j]));
-                buf[n] = acc;
-            }
+            static_assert(MAX_CHANNELS / 2 + 1 <= 5, "sections of a fold");
+            if (cols <= 2 * Lp) fold_channel<2, 8>(qc, buf, srow, preq, cols, Lp, tid, nt);
+            else if (cols <= 3 * Lp) fold_channel<3, 4>(qc, buf, srow, preq, cols, Lp, tid, nt);
+            else fold_channel<5, 2>(qc, buf, srow, preq, cols, Lp, tid, nt);
             __syncthreads();
         }
         // forward DIF, filter multiply fused with the last stage, inverse DIT
