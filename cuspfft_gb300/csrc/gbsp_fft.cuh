@@ -322,6 +322,14 @@ template <int P> struct Radix<P, false> {
 // Thread -> butterfly mapping: for spans m >= 16 consecutive threads take
 // consecutive k (unit-stride shared-memory accesses); for shorter spans with
 // R*m odd they take consecutive j, i.e. stride R*m, which hits distinct banks.
+// PAD: the row buffer has one empty slot after every 2^sh elements (16 or 32),
+// element i at i + (i >> sh).  A span-1 stage of even radix R reads t*R + s,
+// which meets 16/gcd(R, 16) of the 16 eight-byte banks (radix 16: one); with
+// the padding consecutive t step by an odd number of slots (R = 2^sh) or by R
+// with a slot every 16 (R < 16).  It is used where the other stages keep whole
+// aligned groups of 16 lanes together (every span a multiple of the unit, or a
+// power of two below it), so that they stay free of conflicts, and the
+// element offsets s*m keep adding up.
 // `magic` = ceil(2^32/d) gives t/d exactly for t, d < 2^16 where d is m
 // (k-fastest) or l = Lp/(R*m) (j-fastest).
 __host__ __device__ constexpr bool stage_j_fastest(int R, int m, int l) {
@@ -334,15 +342,19 @@ __device__ __forceinline__ V tw_load(const V* __restrict__ p) {
     else return *p;
 }
 
-template <int R, int MODE, bool TWG, typename V>
+template <bool PAD>
+__device__ __forceinline__ int padded(int i, int sh) { return PAD ? i + (i >> sh) : i; }
+
+template <int R, int MODE, bool TWG, bool PAD, typename V>
 __device__ __forceinline__ void fft_stage(V* __restrict__ buf, int Lp, int m, uint32_t magic,
                                           const V* __restrict__ tw, const V* __restrict__ filt,
-                                          int tid, int nthreads) {
+                                          int sh, int tid, int nthreads) {
     using RX = Radix<R>;
     const int nb = Lp / R;
+    auto off = [&](int s) { return padded<PAD>(s * m, sh); };
     if constexpr (MODE == 2) {
         for (int t = tid; t < nb; t += nthreads) {
-            V* p = buf + t * R;
+            V* p = buf + padded<PAD>(t * R, sh);
             V a[R];
 #pragma unroll
             for (int s = 0; s < R; s++) a[s] = p[s];
@@ -363,41 +375,41 @@ __device__ __forceinline__ void fft_stage(V* __restrict__ buf, int Lp, int m, ui
         if (m == 1) { j = t; k = 0; }
         else if (!jfast) { j = (int)__umulhi((uint32_t)t, magic); k = t - j * m; }
         else { k = (int)__umulhi((uint32_t)t, magic); j = t - k * l; }
-        const int base = j * R * m + k;
+        const int base = padded<PAD>(j * R * m + k, sh);
         const V* twk = tw + k;
         V a[R];
         if (MODE == 1) {
             // inputs q sit in register out_reg(q)
 #pragma unroll
-            for (int q = 0; q < R; q++) a[RX::out_reg(q)] = buf[base + q * m];
+            for (int q = 0; q < R; q++) a[RX::out_reg(q)] = buf[base + off(q)];
 #pragma unroll
             for (int q = 1; q < R; q++)
                 a[RX::out_reg(q)] = cmulc(a[RX::out_reg(q)], tw_load<TWG>(twk + (q - 1) * m));
             RX::inv(a);
 #pragma unroll
-            for (int s = 0; s < R; s++) buf[base + s * m] = a[s];
+            for (int s = 0; s < R; s++) buf[base + off(s)] = a[s];
         } else {
 #pragma unroll
-            for (int s = 0; s < R; s++) a[s] = buf[base + s * m];
+            for (int s = 0; s < R; s++) a[s] = buf[base + off(s)];
             RX::fwd(a);
 #pragma unroll
             for (int q = 1; q < R; q++)
                 a[RX::out_reg(q)] = cmul(a[RX::out_reg(q)], tw_load<TWG>(twk + (q - 1) * m));
 #pragma unroll
-            for (int q = 0; q < R; q++) buf[base + q * m] = a[RX::out_reg(q)];
+            for (int q = 0; q < R; q++) buf[base + off(q)] = a[RX::out_reg(q)];
         }
     }
 }
 
 // The first forward stage reading its inputs straight from global memory
-// (the sequential-channel rows: no bulk copy into shared memory, no separate
+// (multi-channel and padded rows: no bulk copy into shared memory, no separate
 // pre-twiddle pass): x[n] = src[n] * pre[n] (PRE) or src[n] for n < cols,
 // zero beyond.  Stage 0 has span m = Lp / R and one block, so butterfly k
 // reads x[k + s*m]; results go to buf in the stage's usual places.
-template <int R, bool PRE, typename V>
+template <int R, bool PRE, bool PAD, typename V>
 __device__ __forceinline__ void fft_stage0_global(V* __restrict__ buf, const V* __restrict__ src,
                                                   const V* __restrict__ pre, int cols, int m,
-                                                  const V* __restrict__ tw, int tid, int nthreads) {
+                                                  const V* __restrict__ tw, int sh, int tid, int nthreads) {
     using RX = Radix<R>;
     for (int k = tid; k < m; k += nthreads) {
         V a[R];
@@ -415,7 +427,7 @@ __device__ __forceinline__ void fft_stage0_global(V* __restrict__ buf, const V* 
 #pragma unroll
         for (int q = 1; q < R; q++) a[RX::out_reg(q)] = cmul(a[RX::out_reg(q)], __ldg(tw + k + (q - 1) * m));
 #pragma unroll
-        for (int q = 0; q < R; q++) buf[k + q * m] = a[RX::out_reg(q)];
+        for (int q = 0; q < R; q++) buf[padded<PAD>(k, sh) + padded<PAD>(q * m, sh)] = a[RX::out_reg(q)];
     }
 }
 
@@ -435,14 +447,14 @@ constexpr int MAX_RADIX_NT512 = 40;
 // Runs one stage of radix R; returns false (and touches nothing) when this
 // kernel was not compiled for R, so a plan/kernel mismatch is reported
 // instead of silently skipping the stage.
-template <int MODE, int MAXR, bool TWG, typename V>
+template <int MODE, int MAXR, bool TWG, bool PAD, typename V>
 __device__ __forceinline__ bool fft_stage_dispatch(int R, V* buf, int Lp, int m, uint32_t magic,
-                                                   const V* tw, const V* filt, int tid, int nthreads) {
+                                                   const V* tw, const V* filt, int sh, int tid, int nthreads) {
     switch (R) {
 #define GBSP_STAGE_CASE(r)                                                                   \
         case r:                                                                              \
             if constexpr (r <= MAXR) {                                                       \
-                fft_stage<r, MODE, TWG>(buf, Lp, m, magic, tw, filt, tid, nthreads);         \
+                fft_stage<r, MODE, TWG, PAD>(buf, Lp, m, magic, tw, filt, sh, tid, nthreads); \
                 return true;                                                                 \
             }                                                                                \
             return false;
@@ -452,14 +464,14 @@ __device__ __forceinline__ bool fft_stage_dispatch(int R, V* buf, int Lp, int m,
     }
 }
 
-template <int MAXR, bool PRE, typename V>
+template <int MAXR, bool PRE, bool PAD, typename V>
 __device__ __forceinline__ bool fft_stage0_global_dispatch(int R, V* buf, const V* src, const V* pre, int cols,
-                                                           int m, const V* tw, int tid, int nthreads) {
+                                                           int m, const V* tw, int sh, int tid, int nthreads) {
     switch (R) {
 #define GBSP_STAGE0_CASE(r)                                                                  \
         case r:                                                                              \
             if constexpr (r <= MAXR) {                                                       \
-                fft_stage0_global<r, PRE>(buf, src, pre, cols, m, tw, tid, nthreads);        \
+                fft_stage0_global<r, PRE, PAD>(buf, src, pre, cols, m, tw, sh, tid, nthreads); \
                 return true;                                                                 \
             }                                                                                \
             return false;

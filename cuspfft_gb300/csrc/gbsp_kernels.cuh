@@ -570,6 +570,7 @@ __device__ __forceinline__ void fold_channel(int q, float2* buf, const float2* x
 //               results wait in an L2-resident scratch for the combine
 //   ROW_SEQW    ROW_SEQ for more than MAX_CHANNELS channels (very wide rows;
 //               a separate instance, so the common one keeps its registers)
+//   (ROW_SINGLE and ROW_DIRECT also come with a padded row buffer, PAD)
 //   ROW_DIRECT  K == 1 and a direct plan (cols smooth: one forward FFT of
 //               length cols, no Bluestein convolution), its own instance so
 //               the Bluestein one keeps its registers
@@ -583,7 +584,9 @@ constexpr int ROW_SINGLE = 0, ROW_CLUSTER = 1, ROW_SEQ = 2, ROW_SEQW = 3, ROW_DI
 // drev in the writer.
 // DIRECT: 0 never (Bluestein), 1 always (ROW_DIRECT), 2 per row from a.drev
 // (the batched kernel, whose matrices mix both kinds)
-template <int MAXR, int MODE, int DIRECT = (MODE == ROW_DIRECT ? 1 : 0)>
+// PAD: the row buffer is padded (fd.sh, see fft_stage); K = 1, and stage 0
+// reads the row from global memory (a bulk copy cannot leave the gaps)
+template <int MAXR, int MODE, bool PAD, int DIRECT = (MODE == ROW_DIRECT ? 1 : 0)>
 __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& fd, int t, int q, float2* buf,
                                               const float2* twr, const float2* const* zsrc, uint64_t* bar,
                                               uint32_t& parity, int& err_bits) {
@@ -599,6 +602,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
     // sit in shared memory
     const float2* tw0 = a.fft_tw + fd.twoff[0];
     auto tw_smem = [&](int s) -> const float2* { return twr + (fd.twoff[s] - fd.rest_base); };
+    const int sh = fd.sh;
     const int u = a.u0 + t;
     const float2* srow = a.S + (size_t)t * a.s_pitch;
     const bool direct = DIRECT == 1 || (DIRECT == 2 && a.drev != nullptr);
@@ -612,7 +616,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
         // network has a separate first stage read the row straight from
         // global memory in that stage, pre-twiddle included
         const int S1 = fd.nst - 1;
-        const bool g0 = (SEQ || CLUSTER) && cols_even <= Lp && S1 > 0;
+        const bool g0 = PAD || ((SEQ || CLUSTER) && cols_even <= Lp && S1 > 0);
         // (a single channel always has cols_even <= Lp: L >= 2*cols - 1)
         if (g0) {
         } else if (!MULTI || cols_even <= Lp) {
@@ -663,31 +667,34 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
         // (a direct plan runs the forward network alone, its last stage --
         // span 1, twiddles exactly 1 -- included: X in digit-reversed order)
         const int S_fwd = direct ? S1 + 1 : S1;
-        if ((SEQ || CLUSTER) && g0) {
-            ok &= (qc == 0) ? fft_stage0_global_dispatch<MAXR, false>(fd.R[0], buf, srow, none, cols, fd.m[0], tw0,
-                                                                       tid, nt)
-                            : fft_stage0_global_dispatch<MAXR, true>(fd.R[0], buf, srow, preq, cols, fd.m[0], tw0,
-                                                                      tid, nt);
+        if ((PAD || SEQ || CLUSTER) && g0) {
+            ok &= (!MULTI || qc == 0)
+                      ? fft_stage0_global_dispatch<MAXR, false, PAD>(fd.R[0], buf, srow, none, cols, fd.m[0], tw0, sh,
+                                                                     tid, nt)
+                      : fft_stage0_global_dispatch<MAXR, true, PAD>(fd.R[0], buf, srow, preq, cols, fd.m[0], tw0, sh,
+                                                                    tid, nt);
             __syncthreads();
         } else if (S_fwd > 0) {
-            ok &= fft_stage_dispatch<0, MAXR, true>(fd.R[0], buf, Lp, fd.m[0], fd.magic[0], tw0, none, tid, nt);
+            ok &= fft_stage_dispatch<0, MAXR, true, PAD>(fd.R[0], buf, Lp, fd.m[0], fd.magic[0], tw0, none, sh, tid,
+                                                        nt);
             __syncthreads();
         }
         for (int s = 1; s < S_fwd; s++) {
-            ok &= fft_stage_dispatch<0, MAXR, false>(fd.R[s], buf, Lp, fd.m[s], fd.magic[s], tw_smem(s), none,
-                                                     tid, nt);
+            ok &= fft_stage_dispatch<0, MAXR, false, PAD>(fd.R[s], buf, Lp, fd.m[s], fd.magic[s], tw_smem(s), none,
+                                                          sh, tid, nt);
             __syncthreads();
         }
         if (direct) continue;
-        ok &= fft_stage_dispatch<2, MAXR, false>(fd.R[S1], buf, Lp, 1, 0u, none, filtq, tid, nt);
+        ok &= fft_stage_dispatch<2, MAXR, false, PAD>(fd.R[S1], buf, Lp, 1, 0u, none, filtq, sh, tid, nt);
         __syncthreads();
         for (int s = S1 - 1; s >= 1; s--) {
-            ok &= fft_stage_dispatch<1, MAXR, false>(fd.R[s], buf, Lp, fd.m[s], fd.magic[s], tw_smem(s), none,
-                                                     tid, nt);
+            ok &= fft_stage_dispatch<1, MAXR, false, PAD>(fd.R[s], buf, Lp, fd.m[s], fd.magic[s], tw_smem(s), none,
+                                                          sh, tid, nt);
             __syncthreads();
         }
         if (S1 > 0) {
-            ok &= fft_stage_dispatch<1, MAXR, true>(fd.R[0], buf, Lp, fd.m[0], fd.magic[0], tw0, none, tid, nt);
+            ok &= fft_stage_dispatch<1, MAXR, true, PAD>(fd.R[0], buf, Lp, fd.m[0], fd.magic[0], tw0, none, sh, tid,
+                                                        nt);
             __syncthreads();
         }
         if (SEQ && qc < K - 1) {  // park the channel for the combine
@@ -729,7 +736,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
                         zv[w][e] = buf[c < 0 ? 0 : __ldg(a.drev + c)];
                     } else {
                         pv[w][e] = (c >= 0) ? __ldg(a.post + c) : make_float2(0.f, 0.f);
-                        zv[w][e] = buf[c < 0 ? 0 : c];
+                        zv[w][e] = buf[c < 0 ? 0 : padded<PAD>(c, sh)];
                     }
                 }
             }
@@ -891,7 +898,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
 // MODE: ROW_SINGLE, ROW_DIRECT, ROW_CLUSTER (launched with a K-CTA cluster
 // dimension), ROW_SEQ or ROW_SEQW; single-channel plans use the ROW_SINGLE
 // (or ROW_DIRECT) instance, which carries no multi-channel code.
-template <int NTMAX, int MODE>
+template <int NTMAX, int MODE, bool PAD = false>
 __global__ void __launch_bounds__(NTMAX, 1) k_bluestein_rows(RowsArgs a, FFTDesc fd, int* err) {
     extern __shared__ float4 smem_raw[];
     __shared__ uint64_t in_bar;
@@ -899,7 +906,7 @@ __global__ void __launch_bounds__(NTMAX, 1) k_bluestein_rows(RowsArgs a, FFTDesc
     // only a direct row can have odd Lp = cols below its even bulk-copy length
     // (a Bluestein row has Lp >= 2 cols - 1 and the multi-channel loads skip
     // the bulk copy when the row does not fit)
-    float2* twr = buf + (MODE == ROW_DIRECT ? row_buf_len(fd.Lp) : fd.Lp);
+    float2* twr = buf + (PAD ? row_buf_slots(fd) : MODE == ROW_DIRECT ? row_buf_len(fd.Lp) : fd.Lp);
     for (int i = threadIdx.x; i < fd.rest_len; i += blockDim.x) twr[i] = a.fft_tw[fd.rest_base + i];
     if (threadIdx.x == 0) mbar_init(&in_bar, 1);
 
@@ -924,7 +931,7 @@ __global__ void __launch_bounds__(NTMAX, 1) k_bluestein_rows(RowsArgs a, FFTDesc
     int err_bits = 0;
     __syncthreads();
     for (int t = cid; t < a.tile_rows; t += ncl)
-        bluestein_row<MAXR, MODE>(a, fd, t, q, buf, twr, zsrc, &in_bar, parity, err_bits);
+        bluestein_row<MAXR, MODE, PAD>(a, fd, t, q, buf, twr, zsrc, &in_bar, parity, err_bits);
     if (err_bits) atomicOr(err, err_bits);
     if (err_bits & ERR_TIMEOUT) {
         // a copy that never signalled may still be in flight: wait once more
@@ -945,7 +952,7 @@ struct RowsBatch {
     FFTDesc fd;
 };
 
-template <int NTMAX>
+template <int NTMAX, bool PAD>
 __global__ void __launch_bounds__(NTMAX, 1)
 k_bluestein_rows_batch(const RowsBatch* __restrict__ descs, const long* __restrict__ row_begin, int nmat,
                        unsigned long long* queue, int* err) {
@@ -982,14 +989,14 @@ k_bluestein_rows_batch(const RowsBatch* __restrict__ descs, const long* __restri
         if (m != loaded) {
             if (threadIdx.x == 0) cur = descs[m];
             __syncthreads();
-            twr = buf + row_buf_len(cur.fd.Lp);
+            twr = buf + row_buf_slots(cur.fd);
             for (int i = threadIdx.x; i < cur.fd.rest_len; i += blockDim.x)
                 twr[i] = cur.a.fft_tw[cur.fd.rest_base + i];
             __syncthreads();
             loaded = m;
         }
-        bluestein_row<MAXR, ROW_SINGLE, 2>(cur.a, cur.fd, (int)(t - row_begin[m]), 0, buf, twr, zsrc, &in_bar, parity,
-                            err_bits);
+        bluestein_row<MAXR, ROW_SINGLE, PAD, 2>(cur.a, cur.fd, (int)(t - row_begin[m]), 0, buf, twr, zsrc, &in_bar,
+                                                parity, err_bits);
     }
     if (err_bits) atomicOr(err, err_bits);
     if (err_bits & ERR_TIMEOUT) mbar_wait_bounded(&in_bar, parity ^ 1u);

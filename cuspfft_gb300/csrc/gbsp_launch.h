@@ -14,6 +14,7 @@
 #include "gbsp_internal.h"
 #include "gbsp_kernels.cuh"
 #include "gbsp_pass1_mma.cuh"
+#include "gbsp_planner.h"
 
 // Returns a GBSP_ERR_* status (with the message recorded) from the calling
 // function when a CUDA runtime call fails.
@@ -65,13 +66,21 @@ int p1_mma_batch_launch(int grid, size_t smem, cudaStream_t st, const P1MmaArgs*
 struct RowsKernel {
     int mode, ntmax, K, nt;
     size_t smem;
+    bool pad;  // padded row buffer (single channel)
 };
 // CTAs (single channel, sequential channels) or clusters resident at once
 int rows_capacity(const RowsKernel& k, int sms, int* cap);
 int rows_launch(const RowsKernel& k, int grid, cudaStream_t st, const RowsArgs& a, const FFTDesc& fd, int* err);
-int rows_batch_blocks_per_sm(int nt, size_t smem, int* nb);
-int rows_batch_launch(int grid, int nt, size_t smem, cudaStream_t st, const RowsBatch* descs, const long* row_begin,
-                      int nmat, unsigned long long* queue, int* err);
+// ... with a padded row buffer (gbsp_rows_pad.cu)
+int rows_capacity_pad(const RowsKernel& k, int sms, int* cap);
+int rows_launch_pad(const RowsKernel& k, int grid, cudaStream_t st, const RowsArgs& a, const FFTDesc& fd, int* err);
+// batches (gbsp_rows_batch.cu, gbsp_rows_batch_pad.cu)
+int rows_batch_blocks_per_sm(const RowBlock& rb, bool pad, size_t smem, int* nb);
+int rows_batch_blocks_per_sm_pad(const RowBlock& rb, size_t smem, int* nb);
+int rows_batch_launch_pad(const RowBlock& rb, int grid, size_t smem, cudaStream_t st, const RowsBatch* descs,
+                          const long* row_begin, int nmat, unsigned long long* queue, int* err);
+int rows_batch_launch(const RowBlock& rb, bool pad, int grid, size_t smem, cudaStream_t st, const RowsBatch* descs,
+                      const long* row_begin, int nmat, unsigned long long* queue, int* err);
 // the multi-channel modes (clusters: gbsp_rows_multi.cu, sequential
 // channels: gbsp_rows_seq.cu); rows_capacity / rows_launch forward to these
 int rows_capacity_multi(const RowsKernel& k, int sms, int* cap);

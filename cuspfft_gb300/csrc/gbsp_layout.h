@@ -46,6 +46,10 @@ struct FFTDesc {
     int twoff[MAX_STAGES];      // stage twiddle offset in the global table (q-major blocks)
     int rest_base;              // first twiddle of stage 1 (stages >= 1 are staged in smem)
     int rest_len;               // twiddles of stages >= 1
+    int sh;                     // row buffer padding: element i sits at i + (i >> sh); 31 = none
 };
+
+// complex slots of a row buffer, padding included
+GBSP_HD inline int row_buf_slots(const FFTDesc& fd) { return row_buf_len(fd.Lp + (fd.Lp >> fd.sh)); }
 
 }  // namespace gbsp

@@ -13,6 +13,7 @@
 #include <mutex>
 #include <numeric>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -66,6 +67,7 @@ struct gbsp_plan_s {
     int p1_grid = 0;
     size_t p1_smem = 0;
     int rows_grid = 0, rows_threads = 1024, rows_ntmax = 1024;
+    int rows_block = 0;              // launched block (choose_row_block); rows_threads is the planned one
     int row_mode = 0;                // gbsp::ROW_SINGLE / ROW_DIRECT / ROW_CLUSTER / ROW_SEQ / ROW_SEQW
     float2* d_zscratch = nullptr;    // ROW_SEQ: rows_grid x (K-1) x Lp channel results
     size_t rows_smem = 0;
@@ -292,7 +294,7 @@ int launch_pass1(const gbsp_plan_s* p, int u0, int n, float2* S, size_t sp, cons
 }
 
 gbsp::RowsKernel rows_kernel(const gbsp_plan_s* p) {
-    return gbsp::RowsKernel{p->row_mode, p->rows_ntmax, p->K, p->rows_threads, p->rows_smem};
+    return gbsp::RowsKernel{p->row_mode, p->rows_ntmax, p->K, p->rows_block, p->rows_smem, p->fd.sh < 31};
 }
 
 gbsp::RowsArgs rows_args(const gbsp_plan_s* p, const float2* S, size_t s_pitch, int u0, int n, void* d_out,
@@ -345,6 +347,12 @@ int rows_prepare(gbsp_plan_s* p, int sms) {
         return set_error(GBSP_ERR_UNSUPPORTED, "more than " + std::to_string(MAX_CHANNELS) +
                                                    " channels need sequential channels (512-thread rows)");
     if (p->row_mode == ROW_SEQ && p->K > MAX_CHANNELS) p->row_mode = ROW_SEQW;
+    p->rows_block = p->rows_threads;
+    if (p->K == 1) {
+        const RowBlock rb = choose_row_block(p->fd, p->rows_threads, p->u_tile / sms);
+        p->rows_block = rb.nt;
+        p->rows_ntmax = rb.ntmax;
+    }
     int cap = 0;
     const int rc = rows_capacity(rows_kernel(p), sms, &cap);
     if (rc) return rc;
@@ -413,9 +421,11 @@ bool mma_choice(const gbsp_plan_s* p, const gbsp_options* o, const int* col_ptr)
 }
 
 // force_p1: 1-based pass-1 shape imposed by a batch (one shape for all its
-// matrices); 0 leaves the choice to the options.
+// matrices); 0 leaves the choice to the options.  batch_rows: Bluestein rows
+// of the whole batch (0: the plan runs alone).
 int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int* sparse_cols,
-               const gbsp_options* o_in, cudaStream_t st, int force_p1 = 0) {
+               const gbsp_options* o_in, cudaStream_t st, int force_p1 = 0,
+               long batch_rows = 0) {
     gbsp_options o = o_in ? *o_in : gbsp_options{};
     if (force_p1) o.pass1_shape = force_p1;
     GB_CUDA(cudaGetDevice(&p->device));
@@ -436,7 +446,8 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
 
     // ---- lengths, channel split, radices and row block
     gbsp::ChannelSplit sp;
-    if ((rc = gbsp::split_channels(p->cols, &o, smem_cap, &sp))) return rc;
+    if ((rc = gbsp::split_channels(p->cols, batch_rows ? batch_rows : gbsp::launch_rows_of(p->rows, &o), &o, smem_cap,
+                                   &sp))) return rc;
     p->L = sp.L;
     p->K = sp.K;
     p->Lp = sp.Lp;
@@ -996,7 +1007,9 @@ struct gbsp_batch_s {
     // Row launches: one per class of matrices that share a block size and a
     // CTAs-per-SM count, so small rows keep the occupancy they have alone.
     struct RowsClass {
-        int nt = 0, grid = 0, begin = 0, end = 0;  // descriptors [begin, end) in queue order
+        gbsp::RowBlock rb{};
+        bool pad = false;
+        int grid = 0, begin = 0, end = 0;  // descriptors [begin, end) in queue order
         size_t smem = 0;
     };
     std::vector<RowsClass> classes;
@@ -1059,7 +1072,7 @@ int batch_launch(gbsp_batch_s* b, cudaStream_t st) {
         if (b->n_fp32 > 0 && (rc = p1b_dispatch(b, false, 0, st))) return rc;
         for (size_t c = 0; c < b->classes.size(); c++) {
             const auto& k = b->classes[c];
-            if ((rc = gbsp::rows_batch_launch(k.grid, k.nt, k.smem, st, b->d_rows + k.begin,
+            if ((rc = gbsp::rows_batch_launch(k.rb, k.pad, k.grid, k.smem, st, b->d_rows + k.begin,
                                               b->d_row_begin + k.begin + c, k.end - k.begin, b->d_queue + 2 + c,
                                               b->d_err)))
                 return rc;
@@ -1133,6 +1146,8 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
     o.rows_threads = 0;
     o.row_table_mode = 0;
     for (int& r : o.radix) r = 0;  // lengths differ across the batch: per-matrix radices
+    long all_rows = 0;
+    for (int i = 0; i < count; i++) all_rows += mats[i].rows / 2 + 1;
     b->plans.assign(count, nullptr);
     for (int i = 0; i < count && rc == GBSP_OK; i++) {
         gbsp_plan_s* p = new (std::nothrow) gbsp_plan_s();
@@ -1142,7 +1157,7 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
         p->nnz = mats[i].nnz;
         p->n_active = mats[i].n_active;
         b->plans[i] = p;
-        rc = plan_build(p, mats[i].col_ptr, mats[i].row_idx, mats[i].sparse_cols, &o, st, b->p1_shape);
+        rc = plan_build(p, mats[i].col_ptr, mats[i].row_idx, mats[i].sparse_cols, &o, st, b->p1_shape, all_rows);
     }
     if (rc) {
         free_batch(b);
@@ -1152,39 +1167,37 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
     // (block size, CTAs per SM), classes with the longest rows first, and by
     // decreasing channel length inside a class.
     std::vector<int> per_sm(count, 0);
+    std::vector<gbsp::RowBlock> rbs(count);
     for (int i = 0; i < count; i++) {
         const gbsp_plan_s* p = b->plans[i];
         if (p->K != 1 || p->rows_threads > 512) {
             b->separate.push_back(i);
             continue;
         }
-        if (gbsp::rows_batch_blocks_per_sm(p->rows_threads, rows_smem_bytes(p->fd), &per_sm[i]) != GBSP_OK ||
-            per_sm[i] < 1) {
+        rbs[i] = gbsp::choose_row_block(p->fd, p->rows_threads, (int)std::min<long>(all_rows / sms, 1 << 20));
+        if (gbsp::rows_batch_blocks_per_sm(rbs[i], p->fd.sh < 31, rows_smem_bytes(p->fd), &per_sm[i]) != GBSP_OK || per_sm[i] < 1) {
             free_batch(b);
             return set_error(GBSP_ERR_UNSUPPORTED, "gbsp_batch_create: batched row kernel does not fit");
         }
         b->order.push_back(i);
     }
+    auto key = [&](int i) { return std::make_tuple(per_sm[i], -rbs[i].nt, rbs[i].ntmax, b->plans[i]->fd.sh < 31); };
     std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) {
-        const gbsp_plan_s *px = b->plans[x], *py = b->plans[y];
-        if (per_sm[x] != per_sm[y]) return per_sm[x] < per_sm[y];
-        if (px->rows_threads != py->rows_threads) return px->rows_threads > py->rows_threads;
-        return px->Lp > py->Lp;
+        return key(x) != key(y) ? key(x) < key(y) : b->plans[x]->Lp > b->plans[y]->Lp;
     });
     const int n = (int)b->order.size();
     for (int k = 0; k < n; k++) {
-        const gbsp_plan_s* p = b->plans[b->order[k]];
         const int m = b->order[k];
-        if (b->classes.empty() || per_sm[b->order[k - 1]] != per_sm[m] ||
-            b->plans[b->order[k - 1]]->rows_threads != p->rows_threads) {
+        if (b->classes.empty() || key(b->order[k - 1]) != key(m)) {
             gbsp_batch_s::RowsClass c;
-            c.nt = p->rows_threads;
+            c.rb = rbs[m];
+            c.pad = b->plans[m]->fd.sh < 31;
             c.grid = per_sm[m] * sms;
             c.begin = k;
             b->classes.push_back(c);
         }
         b->classes.back().end = k + 1;
-        b->classes.back().smem = std::max(b->classes.back().smem, rows_smem_bytes(p->fd));
+        b->classes.back().smem = std::max(b->classes.back().smem, rows_smem_bytes(b->plans[m]->fd));
     }
     const int ncls = (int)b->classes.size();
     if (n > 0) {

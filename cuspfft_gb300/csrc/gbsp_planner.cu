@@ -18,7 +18,23 @@
 namespace gbsp {
 
 // Stage descriptor for a given radix sequence (product must be Lp).
-int build_fft_desc(int Lp, const std::vector<int>& rs, FFTDesc* fd) {
+//
+// Padding (see fft_stage): the last radix a power of two from 4 on, one slot
+// after every max(16, R_last) elements, every span a multiple of that unit or
+// a power of two below 16 that ends a multiple of 16 (so that off(s) adds up).
+static int pad_shift(const FFTDesc& fd) {
+    const int last = fd.R[fd.nst - 1];
+    if (fd.nst < 2 || (last & (last - 1)) || last < 4 || last > 32) return 31;
+    const int unit = std::max(16, last);
+    for (int s = 0; s < fd.nst - 1; s++) {
+        const int m = fd.m[s];
+        if (m % unit == 0) continue;
+        if (unit != 16 || (m & (m - 1)) || (fd.R[s] * m) % 16) return 31;
+    }
+    return unit == 16 ? 4 : 5;
+}
+
+int build_fft_desc(int Lp, const std::vector<int>& rs, FFTDesc* fd, size_t pad_cap) {
     if ((int)rs.size() > MAX_STAGES || rs.empty()) return GBSP_ERR_UNSUPPORTED;
     long prod = 1;
     for (int r : rs) {
@@ -44,13 +60,18 @@ int build_fft_desc(int Lp, const std::vector<int>& rs, FFTDesc* fd) {
     }
     fd->rest_base = (fd->R[0] - 1) * fd->m[0];
     fd->rest_len = off - fd->rest_base;
+    fd->sh = 31;
+    if (pad_cap > 0) {
+        fd->sh = pad_shift(*fd);
+        if (rows_smem_bytes(*fd) > pad_cap) fd->sh = 31;
+    }
     return GBSP_OK;
 }
 
 int fft_tw_count(const FFTDesc& fd) { return fd.rest_base + fd.rest_len; }
 
 size_t rows_smem_bytes(const FFTDesc& fd) {
-    return ((size_t)row_buf_len(fd.Lp) + (size_t)fd.rest_len) * sizeof(float2);
+    return ((size_t)row_buf_slots(fd) + (size_t)fd.rest_len) * sizeof(float2);
 }
 
 // ---- radix planning -------------------------------------------------------
@@ -93,11 +114,14 @@ static std::vector<int> order_radices(std::vector<int> rs) {
 // largest radix a block of the given maximum size can hold in registers
 int max_radix_for(int nt_max) { return nt_max > 512 ? MAX_RADIX_NT1024 : MAX_RADIX_NT512; }
 
-// SM limits the model uses (GB300: 228 KB shared memory, 64K registers, 2048 threads per SM)
+// SM limits the model uses (GB300: 152 SMs; 228 KB shared memory, 64K registers, 2048 threads per SM)
 constexpr size_t kSmemPerSM = 233472;
 constexpr int kRegsPerSM = 65536;
+constexpr int kSMs = 152;
 
-double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct) {
+double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct, bool feature) {
+    const bool padded = fd.sh < 31 && !feature;  // no bank conflicts to count
+    const bool narrow = nt < 256 && !feature;
     double cost = 0.0;
     for (int s = 0; s < fd.nst; s++) {
         const int R = fd.R[s], m = fd.m[s], nb = fd.Lp / R, l = nb / m;
@@ -110,10 +134,18 @@ double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct) {
         // timed matrices 3.4 -> 3.1 %, and on GB300 every x,..,3 plan measured
         // against its replacement was slower (3460^2 10 %, 40421^2 3-smooth 8 %)
         const bool last = s == fd.nst - 1;
-        double per = rounds * R * (R > 32 ? 1.5 : 1.0) * (last && R <= 3 ? 2.0 : 1.0);
-        const bool strided = (m == 1 && R % 2 == 0) ||
-                             (m > 1 && m < 16 && l > 1 && !stage_j_fastest(R, m, l));
-        if (direct && m == 1 && R % 2 == 0) {
+        // Narrow blocks (choose_row_block) hold a large radix's registers
+        // worse: weights fitted on 19 lengths from 210 to 6400 points, the
+        // first pick's mean regret 7.8 -> 1.9 %.  In wide padded plans radix 32
+        // counts 1.2 (8192 points: [32, 16, 16] 177 us, [32, 32, 8] 198).
+        const double big = (R > 32 || (narrow && R == 32)) ? 1.5
+                           : (padded && R == 32)           ? 1.2
+                           : (narrow && R >= 24)           ? 1.1
+                                                           : 1.0;
+        double per = rounds * R * big * (last && R <= 3 ? 2.0 : 1.0);
+        const bool strided = !padded && ((m == 1 && R % 2 == 0) ||
+                             (m > 1 && m < 16 && l > 1 && !stage_j_fastest(R, m, l)));
+        if (direct && !padded && m == 1 && R % 2 == 0) {
             // A span-1 stage of even radix reads buf[t*R + s]: its bank
             // conflicts grow with R's power-of-two part.  Fitted on direct
             // plans only (GB300, 4001 rows, eight candidates each at seven
@@ -131,7 +163,37 @@ double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct) {
     return cost / ctas;
 }
 
-std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_opt, int nt_opt, bool direct) {
+// A short row's stages are latencies (shared-memory round trips, barriers, the
+// L2 reads of stage 0) with little work between; only more rows in flight fill
+// them.  Measured on GB300 (row kernel, us, at 32, 64, 128, 256 threads a row
+// and 128 registers a thread, best of four radix sequences each):
+//   525 points (30001 x 257)     68 100 144 271   2048 (30001, direct) 271 254 268 331
+//   1680 (20001 x 811)          137 131 153 221   2401 (35001 x 1201)  399 380 390 547
+//   3500 (8001, direct)         123  99  90 111   4096 (6007 x 2003)   129 103 100 118
+//   6400 (9001 x 3163)          348 252 219 233   8192 (6007 x 4001)   391 280 227 224
+//   9216 (5501 x 4603)          406 274 213 215   12000 (8001, direct) 909 525 350 276
+// A wider block shortens the row, a narrower one leaves room for more rows and
+// idles fewer threads in a stage's last round; from about 7000 points on
+// shared memory holds too few rows for that to pay.  At 64 registers a thread
+// more rows fit where shared memory allows (2401 points 380 -> 321 us);
+// radix 16 spills there (2048 points [16, 16, 8] 254 -> 261 us).
+constexpr int BLOCK32_POINTS = 700, BLOCK64_POINTS = 3000, BLOCK128_POINTS = 7000, REGS64_RADIX = 15;
+
+RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm) {
+    int rmax = 0;
+    for (int s = 0; s < fd.nst; s++) rmax = std::max(rmax, fd.R[s]);
+    RowBlock b{nt, (rmax > max_radix_for(1024) || nt <= 512) ? 512 : 1024};
+    if (nt != 256 || fd.Lp > BLOCK128_POINTS) return b;
+    b.nt = fd.Lp <= BLOCK32_POINTS ? 32 : fd.Lp <= BLOCK64_POINTS ? 64 : 128;
+    // 512 threads an SM at 128 registers: with fewer rows, wider blocks
+    while (b.nt < nt && rows_per_sm * b.nt < 512) b.nt *= 2;
+    if (b.nt <= 64 && rmax <= REGS64_RADIX && (int)(kSmemPerSM / (rows_smem_bytes(fd) + 1024)) > 512 / b.nt)
+        b.ntmax = 1024;
+    return b;
+}
+
+std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_opt, int nt_opt, bool direct,
+                                    bool single, int rows_per_sm) {
     std::vector<std::vector<int>> cands;
     if (radix_opt && radix_opt[0] > 0) {
         std::vector<int> rs;
@@ -145,7 +207,7 @@ std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_op
     std::vector<RadixPlan> out;
     for (const auto& rs : cands) {
         FFTDesc fd{};
-        if (build_fft_desc(Lp, rs, &fd) != GBSP_OK) continue;
+        if (build_fft_desc(Lp, rs, &fd, single ? smem_cap : 0) != GBSP_OK) continue;
         if (rows_smem_bytes(fd) > smem_cap) continue;
         const int rmax = *std::max_element(rs.begin(), rs.end());
         const int nt_hi = rmax > max_radix_for(1024) ? 512 : 1024;
@@ -157,7 +219,9 @@ std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_op
             RadixPlan rp;
             rp.fd = fd;
             rp.nt = nt;
-            rp.cost = rows_cost(fd, nt, rows_smem_bytes(fd), direct);
+            // at the block it is launched with
+            const int block = single ? choose_row_block(fd, nt, rows_per_sm).nt : nt;
+            rp.cost = rows_cost(fd, block, rows_smem_bytes(fd), direct);
             out.push_back(rp);
         }
     }
@@ -165,7 +229,13 @@ std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_op
     return out;
 }
 
-int split_channels(int cols, const gbsp_options* o, size_t smem_cap, ChannelSplit* out) {
+long launch_rows_of(int rows, const gbsp_options* o) {
+    const int half = rows / 2 + 1;
+    return (o && o->u_tile > 0) ? std::min(o->u_tile, half) : half;
+}
+
+int split_channels(int cols, long rows, const gbsp_options* o, size_t smem_cap, ChannelSplit* out) {
+    const int rows_per_sm = (int)std::min<long>(rows / kSMs, 1 << 20);
     const int policy = (o && o->length_policy) ? o->length_policy : GBSP_LEN_3SMOOTH;
     if (policy != GBSP_LEN_3SMOOTH && policy != GBSP_LEN_7SMOOTH && policy != GBSP_LEN_POW2)
         return set_error(GBSP_ERR_INVALID, "length_policy must be 2, 3 or 7");
@@ -186,7 +256,7 @@ int split_channels(int cols, const gbsp_options* o, size_t smem_cap, ChannelSpli
     // Bluestein convolution, with a quarter of its FFT work and less rounding
     out->direct = 0;
     if (!(o && o->force_bluestein) && channel_fits(cols) && next_smooth(cols, policy) == cols) {
-        auto ranked = rank_radices(cols, smem_cap, o ? o->radix : nullptr, nt_opt, true);
+        auto ranked = rank_radices(cols, smem_cap, o ? o->radix : nullptr, nt_opt, true, true, rows_per_sm);
         if (!ranked.empty()) {
             out->L = cols;
             out->K = 1;
@@ -205,7 +275,7 @@ int split_channels(int cols, const gbsp_options* o, size_t smem_cap, ChannelSpli
     const int kmax = (o && o->channel_mode == 1) ? MAX_CHANNELS : MAX_SEQ_CHANNELS;
     for (int k = 1; k <= kmax; k++) {
         if (L % k || !channel_fits(L / k)) continue;
-        auto ranked = rank_radices((int)(L / k), smem_cap, o ? o->radix : nullptr, nt_opt);
+        auto ranked = rank_radices((int)(L / k), smem_cap, o ? o->radix : nullptr, nt_opt, false, k == 1, rows_per_sm);
         if (ranked.empty()) continue;
         out->K = k;
         out->Lp = (int)(L / k);
@@ -311,7 +381,7 @@ int enumerate_candidates(int rows, int cols, const gbsp_options* base, size_t sm
     if (rows < 1 || cols < 1 || max_rows < 1) return set_error(GBSP_ERR_INVALID, "enumerate_candidates: bad sizes");
     gbsp_options o = base ? *base : gbsp_options{};
     ChannelSplit sp;
-    if (int rc = split_channels(cols, &o, smem_cap, &sp)) return rc;
+    if (int rc = split_channels(cols, launch_rows_of(rows, &o), &o, smem_cap, &sp)) return rc;
     const int tmode = o.row_table_mode;
     std::vector<int> shapes;
     if (o.pass1_shape > 0) {
@@ -357,7 +427,7 @@ int plan_features(int rows, int cols, int n_active, int nnz, const int* col_ptr,
     if (!cand || !f || rows < 1 || cols < 1 || n_active < 0 || nnz < 0 || (n_active > 0 && !col_ptr))
         return set_error(GBSP_ERR_INVALID, "plan_features: bad arguments");
     ChannelSplit sp;
-    if (int rc = split_channels(cols, cand, smem_cap, &sp)) return rc;
+    if (int rc = split_channels(cols, launch_rows_of(rows, cand), cand, smem_cap, &sp)) return rc;
     const RadixPlan& rp = sp.ranked[0];  // radix and rows_threads of cand restrict the ranking to one choice
     const int sh_idx = cand->pass1_shape - 1;
     if (sh_idx < 0 || sh_idx >= N_P1_SHAPES) return set_error(GBSP_ERR_INVALID, "plan_features: pass1_shape unset");
@@ -400,7 +470,7 @@ int plan_features(int rows, int cols, int n_active, int nnz, const int* col_ptr,
                                          65536 / (rp.nt * regs)}));
     // (the Bluestein form of the row model for every plan: the feature the
     // cost model was trained on)
-    f[27] = lg2(rows_cost(fd, rp.nt, rows_smem_bytes(fd)));
+    f[27] = lg2(rows_cost(fd, rp.nt, rows_smem_bytes(fd), false, true));
     // pass-1 shape (the two-level shapes share the slot of their half-table
     // twin: the model never saw them, and they only appear when nothing else fits)
     f[28 + (sh_idx == 6 ? 1 : sh_idx == 7 ? 5 : sh_idx)] = 1.f;

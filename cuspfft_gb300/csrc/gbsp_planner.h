@@ -11,12 +11,23 @@
 namespace gbsp {
 
 // ---- channel FFT
-int build_fft_desc(int Lp, const std::vector<int>& rs, FFTDesc* fd);
+// pad_cap > 0: pad the row buffer where that helps (FFTDesc::sh) and fits in
+// pad_cap bytes
+int build_fft_desc(int Lp, const std::vector<int>& rs, FFTDesc* fd, size_t pad_cap = 0);
 int fft_tw_count(const FFTDesc& fd);
 size_t rows_smem_bytes(const FFTDesc& fd);
 int max_radix_for(int nt_max);  // largest radix a block of at most nt_max threads holds
-// direct: the plan is one forward FFT (no Bluestein convolution)
-double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct = false);
+// direct: the plan is one forward FFT (no Bluestein convolution).  feature:
+// the form the learned cost model was trained on (no padded buffers).
+double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct = false, bool feature = false);
+
+// The block a single-channel row planned for nt threads is launched with, and
+// the compiled block bound of its kernel (512: 128 registers a thread, 1024:
+// 64).  rows_per_sm: rows there are for each SM.
+struct RowBlock {
+    int nt, ntmax;
+};
+RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm);
 
 struct RadixPlan {
     FFTDesc fd{};
@@ -25,9 +36,10 @@ struct RadixPlan {
 };
 // Every (radix sequence, block size) for channel length Lp that fits in
 // smem_cap, cheapest first by rows_cost.  radix_opt (0-terminated, may be
-// null) and nt_opt (0 = automatic: 256 or 512) restrict the set.
+// null) and nt_opt (0 = automatic: 256 or 512) restrict the set; single: K = 1
+// (padded buffers allowed).
 std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_opt, int nt_opt,
-                                    bool direct = false);
+                                    bool direct, bool single, int rows_per_sm);
 
 // Channel split of the length-L convolution: the smallest K (<= MAX_CHANNELS
 // for clusters, MAX_SEQ_CHANNELS for sequential channels)
@@ -37,7 +49,10 @@ struct ChannelSplit {
     int direct = 0;  // 1: one forward FFT of length cols (cols smooth), no Bluestein
     std::vector<RadixPlan> ranked;
 };
-int split_channels(int cols, const gbsp_options* o, size_t smem_cap, ChannelSplit* out);
+// rows: the Bluestein rows of a launch (they decide the block of short rows).
+int split_channels(int cols, long rows, const gbsp_options* o, size_t smem_cap, ChannelSplit* out);
+// ... of a matrix of `rows` rows under options o
+long launch_rows_of(int rows, const gbsp_options* o);
 
 // ---- pass 1 shapes: {rows per lane, window width, twiddle table layout
 // (TAB_FULL, TAB_HALF, TAB_TWO)}

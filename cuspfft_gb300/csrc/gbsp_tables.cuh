@@ -225,7 +225,7 @@ __device__ __forceinline__ float2 chirp_twiddle(long long c, int q, int cols, in
 }
 
 // Direct plans: drev[f] = position of frequency f after the forward DIF
-// network, sum over stages s of digit_s(f) * m_s, where digit_s(f) =
+// network (in the row buffer, padding included): sum over stages s of digit_s(f) * m_s, where digit_s(f) =
 // (f / (R_0 ... R_{s-1})) mod R_s (the stage-s output q lands at q * m_s).
 __global__ void k_digit_rev(int* drev, FFTDesc fd) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -235,7 +235,7 @@ __global__ void k_digit_rev(int* drev, FFTDesc fd) {
         pos += (t % fd.R[s]) * fd.m[s];
         t /= fd.R[s];
     }
-    drev[f] = pos;
+    drev[f] = pos + (pos >> fd.sh);
 }
 
 // exp(-2*pi*i*e/n) for an exactly reduced integer phase e < n

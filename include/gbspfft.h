@@ -94,7 +94,10 @@ typedef struct {
                               longer convolutions split into channels (a thread-block
                               cluster, or one CTA running them in turn)                   */
     int rows_threads;      /* row-kernel block size: 0 = auto, else a multiple of 32
-                              in [64, 1024] (at most 512 when a radix exceeds 16)         */
+                              in [64, 1024] (at most 512 when a radix exceeds 16).
+                              Rows of up to 7000 points planned for 256 threads are
+                              launched in blocks of 32, 64 or 128 when there are
+                              enough of them                                              */
     int row_table_mode;    /* pass-1 twiddle table: 0 = auto, 1 = full circle,
                               2 = half circle, 3 = two-level (W^p = hi[p/256]*lo[p%256],
                               any row count)                                              */
