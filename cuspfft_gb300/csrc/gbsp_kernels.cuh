@@ -92,6 +92,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Programmatic dependent launch.  A kernel launched with the attribute
+// (launch_kernel) may start while the one before it in the stream still runs:
+// it may read the plan's tables, and waits here before it touches anything
+// another kernel writes.  Every kernel of a transform waits (the attribute
+// then chains: when one is complete, all before it are) and lets its
+// successor start as SMs fall free.  Both are no-ops in a plain launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // Pass 1: twiddle sums over each column's nonzero rows, times the chirp.
 //
@@ -398,8 +407,10 @@ __global__ void __launch_bounds__(P1_THREADS, 1) k_twiddle_sum(P1Args a) {
     float2* stage = reinterpret_cast<float2*>(smem_raw);
     NzInfo* info_all = reinterpret_cast<NzInfo*>(stage + (size_t)32 * KU * p1_pitch(a.cw));
     float2* tab = reinterpret_cast<float2*>(info_all + P1_WARPS * 32);
+    pdl_trigger();
     for (int i = threadIdx.x; i < a.ntab; i += blockDim.x) tab[i] = a.row_tab[i];
     if (threadIdx.x == 0) sh.next_task = 0;
+    pdl_wait();
     // Items are handed out one at a time from a device counter, so CTAs
     // whose windows hold fewer nonzeros take more items and all finish
     // together.  p1_item ends on a barrier, so thread 0 rewrites sh.item only
@@ -427,11 +438,13 @@ __global__ void __launch_bounds__(P1_THREADS, 1) k_twiddle_sum(P1Args a) {
 // each matrix, item_begin[nmat] = total) handed out by a device work queue,
 // one item per grab.  Items are grabbed in increasing order, so a CTA moves
 // forward through the matrices and reloads the twiddle table only when it
-// enters a new one.  *queue must be 0 at launch.
+// enters a new one.  *queue must be 0 at launch.  late: the kernel before it in
+// the stream is independent (the tensor-core part of pass 1), so only the
+// kernel's end waits for it.
 template <typename IDX, int TAB, bool BIG, int KU, bool EXACT>
 __global__ void __launch_bounds__(P1_THREADS, 1)
 k_twiddle_sum_batch(const P1Args* __restrict__ args, const long* __restrict__ item_begin, int nmat,
-                    unsigned long long* queue) {
+                    unsigned long long* queue, int late) {
     extern __shared__ float4 smem_raw[];
     __shared__ P1Shared sh;
     __shared__ P1Args cur;
@@ -439,7 +452,9 @@ k_twiddle_sum_batch(const P1Args* __restrict__ args, const long* __restrict__ it
     __shared__ int s_m;
     float2* stage = reinterpret_cast<float2*>(smem_raw);
     int loaded = -1;
+    pdl_trigger();
     if (threadIdx.x == 0) { sh.next_task = 0; s_m = 0; }
+    if (!late) pdl_wait();
     __syncthreads();
     const long total = item_begin[nmat];
     for (;;) {
@@ -467,6 +482,7 @@ k_twiddle_sum_batch(const P1Args* __restrict__ args, const long* __restrict__ it
         float2* tab = reinterpret_cast<float2*>(info_all + P1_WARPS * 32);
         p1_item<IDX, TAB, BIG, KU, EXACT>(cur, it - item_begin[m], stage, info_all, tab, sh);
     }
+    if (late && blockIdx.x == 0) pdl_wait();
 }
 
 // ---------------------------------------------------------------------------
@@ -527,9 +543,9 @@ struct RowsArgs {
 // U slots a pass, all their loads (L2) issued before any product: one slot a
 // pass waited out the L2 latency Lp / nt times per channel, 46 % of the row
 // kernel on 40421 columns (three channels of 27000, two sections).
-template <bool PRE, int NS, int U>
+template <bool PRE, bool PAD, int NS, int U>
 __device__ __forceinline__ void fold_sections(float2* __restrict__ buf, const float2* __restrict__ x,
-                                              const float2* __restrict__ pre, int cols, int Lp, int tid, int nt) {
+                                              const float2* __restrict__ pre, int cols, int Lp, int sh, int tid, int nt) {
     float2 wk[NS];
 #pragma unroll
     for (int j = 1; j < NS; j++) wk[j] = (PRE && j * Lp < cols) ? __ldg(pre + j * Lp) : make_float2(1.f, 0.f);
@@ -551,15 +567,15 @@ __device__ __forceinline__ void fold_sections(float2* __restrict__ buf, const fl
 #pragma unroll
             for (int j = 1; j < NS; j++) acc = cadd(acc, PRE ? cmul(xv[w][j], wk[j]) : xv[w][j]);
             if (PRE) acc = cmul(acc, pv[w]);
-            if (n0 + w * nt < Lp) buf[n0 + w * nt] = acc;
+            if (n0 + w * nt < Lp) buf[padded<PAD>(n0 + w * nt, sh)] = acc;
         }
     }
 }
-template <int NS, int U>
+template <bool PAD, int NS, int U>
 __device__ __forceinline__ void fold_channel(int q, float2* buf, const float2* x, const float2* pre, int cols, int Lp,
-                                             int tid, int nt) {
-    if (q == 0) fold_sections<false, NS, U>(buf, x, pre, cols, Lp, tid, nt);
-    else fold_sections<true, NS, U>(buf, x, pre, cols, Lp, tid, nt);
+                                             int sh, int tid, int nt) {
+    if (q == 0) fold_sections<false, PAD, NS, U>(buf, x, pre, cols, Lp, sh, tid, nt);
+    else fold_sections<true, PAD, NS, U>(buf, x, pre, cols, Lp, sh, tid, nt);
 }
 
 // How the K channels of a long row are laid out on the GPU.
@@ -568,13 +584,15 @@ __device__ __forceinline__ void fold_channel(int q, float2* buf, const float2* x
 //               cluster; the output combine reads the peers' buffers (DSMEM)
 //   ROW_SEQ     one CTA runs the K channels one after another; the first K-1
 //               results wait in an L2-resident scratch for the combine
+//   ROW_SEQ2    ROW_SEQ for two channels that hold the whole row (no fold; a
+//               separate instance for its registers)
 //   ROW_SEQW    ROW_SEQ for more than MAX_CHANNELS channels (very wide rows;
 //               a separate instance, so the common one keeps its registers)
-//   (ROW_SINGLE and ROW_DIRECT also come with a padded row buffer, PAD)
+//   (all but ROW_CLUSTER and ROW_SEQW also come with a padded row buffer, PAD)
 //   ROW_DIRECT  K == 1 and a direct plan (cols smooth: one forward FFT of
 //               length cols, no Bluestein convolution), its own instance so
 //               the Bluestein one keeps its registers
-constexpr int ROW_SINGLE = 0, ROW_CLUSTER = 1, ROW_SEQ = 2, ROW_SEQW = 3, ROW_DIRECT = 4;
+constexpr int ROW_SINGLE = 0, ROW_CLUSTER = 1, ROW_SEQ = 2, ROW_SEQW = 3, ROW_DIRECT = 4, ROW_SEQ2 = 5;
 
 // One Bluestein row t of the tile (u = u0 + t), channel q of K: input,
 // forward network, filter, inverse network, Hermitian-paired output.  Whole
@@ -584,15 +602,19 @@ constexpr int ROW_SINGLE = 0, ROW_CLUSTER = 1, ROW_SEQ = 2, ROW_SEQW = 3, ROW_DI
 // drev in the writer.
 // DIRECT: 0 never (Bluestein), 1 always (ROW_DIRECT), 2 per row from a.drev
 // (the batched kernel, whose matrices mix both kinds)
-// PAD: the row buffer is padded (fd.sh, see fft_stage); K = 1, and stage 0
-// reads the row from global memory (a bulk copy cannot leave the gaps)
+// PAD: the row buffer is padded (fd.sh, see fft_stage); a single channel's
+// stage 0 then reads the row from global memory (a bulk copy cannot leave the
+// gaps)
 template <int MAXR, int MODE, bool PAD, int DIRECT = (MODE == ROW_DIRECT ? 1 : 0)>
 __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& fd, int t, int q, float2* buf,
                                               const float2* twr, const float2* const* zsrc, uint64_t* bar,
                                               uint32_t& parity, int& err_bits) {
     constexpr bool CLUSTER = MODE == ROW_CLUSTER;
-    constexpr bool MULTI = MODE == ROW_CLUSTER || MODE == ROW_SEQ || MODE == ROW_SEQW;
-    constexpr bool SEQ = MODE == ROW_SEQ || MODE == ROW_SEQW;
+    constexpr bool TWO = MODE == ROW_SEQ2;
+    constexpr bool SEQ = MODE == ROW_SEQ || MODE == ROW_SEQW || TWO;
+    constexpr bool MULTI = CLUSTER || SEQ;
+    // stage 0 reads the row from global memory whatever its length
+    constexpr bool G0 = TWO || (PAD && !MULTI);
     const int tid = threadIdx.x, nt = blockDim.x;
     const int Lp = fd.Lp, K = a.K, cols = a.cols;
     const int half_slots = (int)(a.out_pitch >> 1);
@@ -616,10 +638,10 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
         // network has a separate first stage read the row straight from
         // global memory in that stage, pre-twiddle included
         const int S1 = fd.nst - 1;
-        const bool g0 = PAD || ((SEQ || CLUSTER) && cols_even <= Lp && S1 > 0);
+        const bool g0 = G0 || (MULTI && cols_even <= Lp && S1 > 0);
         // (a single channel always has cols_even <= Lp: L >= 2*cols - 1)
-        if (g0) {
-        } else if (!MULTI || cols_even <= Lp) {
+        if (G0 || g0) {
+        } else if (!PAD && (!MULTI || cols_even <= Lp)) {
             if (tid == 0) {
                 fence_proxy_async_smem();
                 mbar_expect_tx(bar, (uint32_t)cols_even * 8u);
@@ -648,7 +670,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
                 buf[n] = acc;
             }
             __syncthreads();
-        } else if constexpr (MULTI) {
+        } else if constexpr (MULTI && !TWO) {
             // Several input columns fold onto one slot.  Every channel reads
             // the whole S row, so it is loaded to stay in L2 for the next
             // channel (an evict-first load made each channel re-read it from
@@ -657,9 +679,9 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
             // L = K*Lp >= 2*cols - 1 gives cols/Lp <= K/2 + 1/(2Lp): at most
             // K/2 + 1 sections
             static_assert(MAX_CHANNELS / 2 + 1 <= 5, "sections of a fold");
-            if (cols <= 2 * Lp) fold_channel<2, 8>(qc, buf, srow, preq, cols, Lp, tid, nt);
-            else if (cols <= 3 * Lp) fold_channel<3, 4>(qc, buf, srow, preq, cols, Lp, tid, nt);
-            else fold_channel<5, 2>(qc, buf, srow, preq, cols, Lp, tid, nt);
+            if (cols <= 2 * Lp) fold_channel<PAD, 2, 8>(qc, buf, srow, preq, cols, Lp, sh, tid, nt);
+            else if (cols <= 3 * Lp) fold_channel<PAD, 3, 4>(qc, buf, srow, preq, cols, Lp, sh, tid, nt);
+            else fold_channel<PAD, 5, 2>(qc, buf, srow, preq, cols, Lp, sh, tid, nt);
             __syncthreads();
         }
         // forward DIF, filter multiply fused with the last stage, inverse DIT
@@ -667,7 +689,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
         // (a direct plan runs the forward network alone, its last stage --
         // span 1, twiddles exactly 1 -- included: X in digit-reversed order)
         const int S_fwd = direct ? S1 + 1 : S1;
-        if ((PAD || SEQ || CLUSTER) && g0) {
+        if ((G0 || MULTI) && g0) {
             ok &= (!MULTI || qc == 0)
                       ? fft_stage0_global_dispatch<MAXR, false, PAD>(fd.R[0], buf, srow, none, cols, fd.m[0], tw0, sh,
                                                                      tid, nt)
@@ -699,7 +721,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
         }
         if (SEQ && qc < K - 1) {  // park the channel for the combine
             float2* dst = a.zscratch + ((size_t)blockIdx.x * (K - 1) + qc) * Lp;
-            for (int i = tid; i < Lp; i += nt) dst[i] = buf[i];
+            for (int i = tid; i < Lp; i += nt) dst[i] = buf[padded<PAD>(i, sh)];
             __syncthreads();
         }
     }  // channels
@@ -767,7 +789,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
         // rather than once per value.  The channels are summed in order.
         constexpr int WS = 4;
         const float2* zs0 = a.zscratch + (size_t)blockIdx.x * (K - 1) * Lp;
-        if (K == 2) {
+        if (TWO || K == 2) {
             // Two channels (Lp >= cols, so both read slot c itself): all of
             // a pass's loads are issued before any product, with no channel
             // loop and no wrap of c; the sum runs in the general order.
@@ -787,7 +809,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
                         pa[w][e] = __ldg(p0 + c);
                         za[w][e] = __ldcg(zs0 + c);
                         pb[w][e] = __ldg(p1 + c);
-                        zb[w][e] = buf[c];
+                        zb[w][e] = buf[padded<PAD>(c, sh)];
                     }
                 }
 #pragma unroll
@@ -810,7 +832,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
                     __stcs(dst, make_float4(o[0].x, o[0].y, o[1].x, o[1].y));
                 }
             }
-        } else
+        } else if constexpr (!TWO)
         for (int s0 = lo + tid; s0 < hi; s0 += WS * nt) {
             int cc[WS][2], nn[WS][2];
             float2 acc[WS][2];
@@ -840,7 +862,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
                         pv[w][e] = __ldg(pq + cc[w][e]);
-                        zv[w][e] = last ? buf[nn[w][e]] : __ldcg(zq + nn[w][e]);
+                        zv[w][e] = last ? buf[padded<PAD>(nn[w][e], sh)] : __ldcg(zq + nn[w][e]);
                     }
 #pragma unroll
                 for (int w = 0; w < WS; w++)
@@ -896,7 +918,7 @@ __device__ __forceinline__ void bluestein_row(const RowsArgs& a, const FFTDesc& 
 }
 
 // MODE: ROW_SINGLE, ROW_DIRECT, ROW_CLUSTER (launched with a K-CTA cluster
-// dimension), ROW_SEQ or ROW_SEQW; single-channel plans use the ROW_SINGLE
+// dimension), ROW_SEQ, ROW_SEQ2 or ROW_SEQW; single-channel plans use the ROW_SINGLE
 // (or ROW_DIRECT) instance, which carries no multi-channel code.
 template <int NTMAX, int MODE, bool PAD = false>
 __global__ void __launch_bounds__(NTMAX, 1) k_bluestein_rows(RowsArgs a, FFTDesc fd, int* err) {
@@ -907,8 +929,10 @@ __global__ void __launch_bounds__(NTMAX, 1) k_bluestein_rows(RowsArgs a, FFTDesc
     // (a Bluestein row has Lp >= 2 cols - 1 and the multi-channel loads skip
     // the bulk copy when the row does not fit)
     float2* twr = buf + (PAD ? row_buf_slots(fd) : MODE == ROW_DIRECT ? row_buf_len(fd.Lp) : fd.Lp);
+    pdl_trigger();
     for (int i = threadIdx.x; i < fd.rest_len; i += blockDim.x) twr[i] = a.fft_tw[fd.rest_base + i];
     if (threadIdx.x == 0) mbar_init(&in_bar, 1);
+    pdl_wait();
 
     constexpr int MAXR = (NTMAX > 512) ? MAX_RADIX_NT1024 : MAX_RADIX_NT512;
     int q = 0, cid = blockIdx.x, ncl = gridDim.x;
@@ -946,7 +970,10 @@ __global__ void __launch_bounds__(NTMAX, 1) k_bluestein_rows(RowsArgs a, FFTDesc
 // matrices in order and reloads the matrix's descriptor and stage twiddles
 // only when it moves to the next one.  Shared memory holds the largest
 // matrix's row buffer plus its stage twiddles (the twiddles of each matrix
-// sit right after its own row buffer).  *queue must be 0 at launch.
+// sit right after its own row buffer).  *queue must be 0 at launch.  late: the
+// kernel before it in the stream is the rows of another class, which started
+// after pass 1 was complete; only the kernel's end waits for it, so that its
+// blocks fill the SMs the other class leaves.
 struct RowsBatch {
     RowsArgs a;
     FFTDesc fd;
@@ -955,7 +982,7 @@ struct RowsBatch {
 template <int NTMAX, bool PAD>
 __global__ void __launch_bounds__(NTMAX, 1)
 k_bluestein_rows_batch(const RowsBatch* __restrict__ descs, const long* __restrict__ row_begin, int nmat,
-                       unsigned long long* queue, int* err) {
+                       unsigned long long* queue, int late, int* err) {
     extern __shared__ float4 smem_raw[];
     __shared__ uint64_t in_bar;
     __shared__ RowsBatch cur;
@@ -973,6 +1000,9 @@ k_bluestein_rows_batch(const RowsBatch* __restrict__ descs, const long* __restri
     int err_bits = 0;
     int loaded = -1;
     const long total = row_begin[nmat];
+    // the successor may start once pass 1 is known to be complete
+    if (!late) pdl_wait();
+    pdl_trigger();
     __syncthreads();
     for (;;) {
         if (threadIdx.x == 0) {
@@ -998,6 +1028,7 @@ k_bluestein_rows_batch(const RowsBatch* __restrict__ descs, const long* __restri
         bluestein_row<MAXR, ROW_SINGLE, PAD, 2>(cur.a, cur.fd, (int)(t - row_begin[m]), 0, buf, twr, zsrc, &in_bar,
                                                 parity, err_bits);
     }
+    if (late && blockIdx.x == 0) pdl_wait();
     if (err_bits) atomicOr(err, err_bits);
     if (err_bits & ERR_TIMEOUT) mbar_wait_bounded(&in_bar, parity ^ 1u);
 }

@@ -10,8 +10,9 @@ int p1_blocks_per_sm(const P1Kernel& k, size_t smem, int* nb) {
     return k.exact ? Pass1Set<true>::blocks(k, smem, nb) : Pass1Set<false>::blocks(k, smem, nb);
 }
 
-int p1_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, const P1Args& a) {
-    return k.exact ? Pass1Set<true>::launch(k, grid, smem, st, a) : Pass1Set<false>::launch(k, grid, smem, st, a);
+int p1_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, bool pdl, const P1Args& a) {
+    return k.exact ? Pass1Set<true>::launch(k, grid, smem, st, pdl, a)
+                   : Pass1Set<false>::launch(k, grid, smem, st, pdl, a);
 }
 
 int p1_batch_blocks_per_sm(const P1Kernel& k, size_t smem, int* nb) {
@@ -19,9 +20,9 @@ int p1_batch_blocks_per_sm(const P1Kernel& k, size_t smem, int* nb) {
 }
 
 int p1_batch_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, const P1Args* args,
-                    const long* item_begin, int nmat, unsigned long long* queue) {
-    return k.exact ? Pass1Set<true>::batch_launch(k, grid, smem, st, args, item_begin, nmat, queue)
-                   : Pass1Set<false>::batch_launch(k, grid, smem, st, args, item_begin, nmat, queue);
+                    const long* item_begin, int nmat, unsigned long long* queue, bool late) {
+    return k.exact ? Pass1Set<true>::batch_launch(k, grid, smem, st, args, item_begin, nmat, queue, late)
+                   : Pass1Set<false>::batch_launch(k, grid, smem, st, args, item_begin, nmat, queue, late);
 }
 
 }  // namespace gbsp

@@ -19,9 +19,8 @@ struct P1Ops {
         GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, kern, P1_THREADS, smem));
         return GBSP_OK;
     }
-    static int launch(int grid, size_t smem, cudaStream_t st, const P1Args& a) {
-        k_twiddle_sum<IDX, TAB, BIG, KU, EXACT><<<grid, P1_THREADS, smem, st>>>(a);
-        GB_CUDA(cudaGetLastError());
+    static int launch(int grid, size_t smem, cudaStream_t st, bool pdl, const P1Args& a) {
+        GB_CUDA(launch_kernel(k_twiddle_sum<IDX, TAB, BIG, KU, EXACT>, grid, P1_THREADS, smem, st, pdl, 1, a));
         return GBSP_OK;
     }
     static int batch_blocks(size_t smem, int* nb) {
@@ -31,9 +30,9 @@ struct P1Ops {
         return GBSP_OK;
     }
     static int batch_launch(int grid, size_t smem, cudaStream_t st, const P1Args* args, const long* item_begin,
-                            int nmat, unsigned long long* queue) {
-        k_twiddle_sum_batch<IDX, TAB, BIG, KU, EXACT><<<grid, P1_THREADS, smem, st>>>(args, item_begin, nmat, queue);
-        GB_CUDA(cudaGetLastError());
+                            int nmat, unsigned long long* queue, bool late) {
+        GB_CUDA(launch_kernel(k_twiddle_sum_batch<IDX, TAB, BIG, KU, EXACT>, grid, P1_THREADS, smem, st, late, 1, args,
+                              item_begin, nmat, queue, (int)late));
         return GBSP_OK;
     }
 };
@@ -64,16 +63,16 @@ struct Pass1Set {
     static int blocks(const P1Kernel& k, size_t smem, int* nb) {
         return with_p1<EXACT>(k, [&](auto ops) { return decltype(ops)::blocks(smem, nb); });
     }
-    static int launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, const P1Args& a) {
-        return with_p1<EXACT>(k, [&](auto ops) { return decltype(ops)::launch(grid, smem, st, a); });
+    static int launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, bool pdl, const P1Args& a) {
+        return with_p1<EXACT>(k, [&](auto ops) { return decltype(ops)::launch(grid, smem, st, pdl, a); });
     }
     static int batch_blocks(const P1Kernel& k, size_t smem, int* nb) {
         return with_p1<EXACT>(k, [&](auto ops) { return decltype(ops)::batch_blocks(smem, nb); });
     }
     static int batch_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, const P1Args* args,
-                            const long* item_begin, int nmat, unsigned long long* queue) {
+                            const long* item_begin, int nmat, unsigned long long* queue, bool late) {
         return with_p1<EXACT>(k, [&](auto ops) {
-            return decltype(ops)::batch_launch(grid, smem, st, args, item_begin, nmat, queue);
+            return decltype(ops)::batch_launch(grid, smem, st, args, item_begin, nmat, queue, late);
         });
     }
 };

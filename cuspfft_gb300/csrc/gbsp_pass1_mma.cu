@@ -13,10 +13,9 @@ int p1_mma_prepare(size_t smem, bool batch) {
     return GBSP_OK;
 }
 
-int p1_mma_launch(int sms, size_t smem, cudaStream_t st, const P1MmaArgs& a) {
+int p1_mma_launch(int sms, size_t smem, cudaStream_t st, bool pdl, const P1MmaArgs& a) {
     const int grid = (int)std::min<long>(sms, p1_mma_items(a));
-    k_twiddle_mma<false><<<grid, MM_THREADS, smem, st>>>(a, nullptr, nullptr, 1, a.queue);
-    GB_CUDA(cudaGetLastError());
+    GB_CUDA(launch_kernel(k_twiddle_mma<false>, grid, MM_THREADS, smem, st, pdl, 1, a, nullptr, nullptr, 1, a.queue));
     return GBSP_OK;
 }
 

@@ -400,6 +400,7 @@ k_twiddle_mma(P1MmaArgs one, const P1MmaArgs* __restrict__ args, const long* __r
             tab[mm_slot(i)] = w;
         }
     };
+    pdl_trigger();
     if (!BATCH) load_table(one, threadIdx.x, MM_THREADS);
     for (int i = threadIdx.x; i < (int)((sizeof(sh.desc) + sizeof(sh.item)) / 4); i += MM_THREADS)
         reinterpret_cast<int*>(&sh)[i] = 0;
@@ -421,6 +422,7 @@ k_twiddle_mma(P1MmaArgs one, const P1MmaArgs* __restrict__ args, const long* __r
     }
     if (warp == MM_ISSUER) tc::alloc(&sh.tmem, MM_TMEM_COLS);
     tc::fence_before();
+    pdl_wait();
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = sh.tmem;

@@ -68,7 +68,7 @@ struct gbsp_plan_s {
     size_t p1_smem = 0;
     int rows_grid = 0, rows_threads = 1024, rows_ntmax = 1024;
     int rows_block = 0;              // launched block (choose_row_block); rows_threads is the planned one
-    int row_mode = 0;                // gbsp::ROW_SINGLE / ROW_DIRECT / ROW_CLUSTER / ROW_SEQ / ROW_SEQW
+    int row_mode = 0;                // gbsp::ROW_*
     float2* d_zscratch = nullptr;    // ROW_SEQ: rows_grid x (K-1) x Lp channel results
     size_t rows_smem = 0;
     size_t device_bytes = 0;
@@ -207,6 +207,11 @@ void free_plan(gbsp_plan_s* p) {
     delete p;
 }
 
+// one CTA runs the channels in turn (and parks them in the plan's scratch)
+bool seq_channels(const gbsp_plan_s* p) {
+    return p->row_mode == gbsp::ROW_SEQ || p->row_mode == gbsp::ROW_SEQ2 || p->row_mode == gbsp::ROW_SEQW;
+}
+
 inline unsigned blocks_for(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 gbsp::P1Kernel p1_kernel(const gbsp_plan_s* p) {
@@ -287,10 +292,10 @@ constexpr long long MMA_MIN_ROWS_PER_COL = 10000;  // rows x nonzeros per column
 
 // chirp == nullptr gives the raw column sums (gbsp_column_sums)
 int launch_pass1(const gbsp_plan_s* p, int u0, int n, float2* S, size_t sp, const float2* chirp,
-                 cudaStream_t st) {
+                 cudaStream_t st, bool pdl = false) {
     if (p->mma && n >= MMA_MIN_ROWS)
-        return gbsp::p1_mma_launch(p->sms, p->mma_smem, st, p1_mma_args(p, u0, n, S, sp, chirp));
-    return gbsp::p1_launch(p1_kernel(p), p->p1_grid, p->p1_smem, st, p1_args(p, u0, n, S, sp, chirp));
+        return gbsp::p1_mma_launch(p->sms, p->mma_smem, st, pdl, p1_mma_args(p, u0, n, S, sp, chirp));
+    return gbsp::p1_launch(p1_kernel(p), p->p1_grid, p->p1_smem, st, pdl, p1_args(p, u0, n, S, sp, chirp));
 }
 
 gbsp::RowsKernel rows_kernel(const gbsp_plan_s* p) {
@@ -323,12 +328,13 @@ gbsp::RowsArgs rows_args(const gbsp_plan_s* p, const float2* S, size_t s_pitch, 
 
 // the row kernel with fully specified arguments (input tile, output slab
 // and row map)
-int launch_rows_args(const gbsp_plan_s* p, const gbsp::RowsArgs& a, cudaStream_t st) {
-    return gbsp::rows_launch(rows_kernel(p), p->rows_grid, st, a, p->fd, p->d_err);
+int launch_rows_args(const gbsp_plan_s* p, const gbsp::RowsArgs& a, cudaStream_t st, bool pdl = false) {
+    return gbsp::rows_launch(rows_kernel(p), p->rows_grid, st, pdl, a, p->fd, p->d_err);
 }
 
-int launch_rows(const gbsp_plan_s* p, int u0, int n, void* d_out, size_t out_pitch, cudaStream_t st) {
-    return launch_rows_args(p, rows_args(p, p->d_S, p->s_pitch, u0, n, d_out, out_pitch), st);
+int launch_rows(const gbsp_plan_s* p, int u0, int n, void* d_out, size_t out_pitch, cudaStream_t st,
+                bool pdl = false) {
+    return launch_rows_args(p, rows_args(p, p->d_S, p->s_pitch, u0, n, d_out, out_pitch), st, pdl);
 }
 
 // Block size and radices are already chosen; pick the compiled variant and
@@ -347,6 +353,11 @@ int rows_prepare(gbsp_plan_s* p, int sms) {
         return set_error(GBSP_ERR_UNSUPPORTED, "more than " + std::to_string(MAX_CHANNELS) +
                                                    " channels need sequential channels (512-thread rows)");
     if (p->row_mode == ROW_SEQ && p->K > MAX_CHANNELS) p->row_mode = ROW_SEQW;
+    if (p->row_mode == ROW_SEQ && p->K == 2 && ((p->cols + 1) & ~1) <= p->Lp && p->fd.nst > 1) p->row_mode = ROW_SEQ2;
+    if (p->row_mode == ROW_CLUSTER || p->row_mode == ROW_SEQW) {  // not compiled with padding
+        p->fd.sh = 31;
+        p->rows_smem = rows_smem_bytes(p->fd);
+    }
     p->rows_block = p->rows_threads;
     if (p->K == 1) {
         const RowBlock rb = choose_row_block(p->fd, p->rows_threads, p->u_tile / sms);
@@ -483,6 +494,18 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
     {
         const std::vector<int> fit = gbsp::fitting_p1_shapes(p->rows, smem_cap, tmode);
         int idx = fit.empty() ? -1 : fit[0];
+        // Tiles of at most 128 rows (the reference's default u_tile) fill half
+        // of a 256-row item: 128-row shapes instead, with 64-column windows
+        // where there are enough.  Pass 1 of all tiles of 128 rows, 256-row
+        // shape against 128-row ones with 64- and 32-column windows: 8219^2
+        // 1.16 ms, 0.83, 0.90; 16706^2 3.35, 2.45, 2.60; 3001 x 2048 0.175,
+        // 0.196, 0.149.
+        if (p->u_tile <= 128 && p->half_rows > 128)
+            for (int i : {p->cols >= 4096 ? 2 : 5, 5})
+                if (std::find(fit.begin(), fit.end(), i) != fit.end()) {
+                    idx = i;
+                    break;
+                }
         if (o.pass1_shape > 0) {
             idx = o.pass1_shape - 1;
             if (std::find(fit.begin(), fit.end(), idx) == fit.end())
@@ -556,7 +579,7 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
                                 (size_t)K * cols * sizeof(float2), (size_t)K * Lp * sizeof(float2),
                                 (size_t)ntw * sizeof(float2), (size_t)K * Lp * sizeof(double2),
                                 (size_t)K * Lp * sizeof(double2), s_bytes, staging,
-                                (p->row_mode == gbsp::ROW_SEQ || p->row_mode == gbsp::ROW_SEQW)
+                                seq_channels(p)
                                     ? (size_t)p->rows_grid * (K - 1) * Lp * sizeof(float2)
                                     : 0,
                                 stream_slab, stream_slab, p->direct ? (size_t)Lp * sizeof(int) : 0, kptr_bytes,
@@ -598,7 +621,7 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
         // no setup of its own
         if ((rc = stream_objects(p))) return rc;
     }
-    if ((p->row_mode == gbsp::ROW_SEQ || p->row_mode == gbsp::ROW_SEQW) &&
+    if (seq_channels(p) &&
         (rc = dev_alloc(p, (void**)&p->d_zscratch, (size_t)p->rows_grid * (K - 1) * Lp * sizeof(float2))))
         return rc;
     if ((rc = dev_alloc(p, &p->d_row_idx, (size_t)std::max(p->nnz, 1) * p->idx_bytes))) return rc;
@@ -761,6 +784,12 @@ int check_out(const gbsp_plan_s* p, const void* d_out, size_t out_pitch, const c
 
 }  // namespace
 
+// Row launches of up to this many points start while pass 1 ends (saves ~3 us
+// each: 301 x 257 21.5 -> 15.8 us with both launches); longer ones after it, as
+// they ran slower so (16706^2 3132 -> 3305 us, 8219^2 884 -> 890: pass 1 leaves
+// the SM set for its own shared-memory size).
+static constexpr long PDL_ROWS_POINTS = 32l << 20;
+
 extern "C" {
 
 int gbsp_plan_create(int rows, int cols, int n_active, int nnz, const int* col_ptr,
@@ -845,8 +874,8 @@ int gbsp_execute(gbsp_plan_t p, void* d_out, size_t out_pitch, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     for (int u0 = 0; u0 < p->half_rows; u0 += p->u_tile) {
         const int n = std::min(p->u_tile, p->half_rows - u0);
-        if ((rc = launch_pass1(p, u0, n, p->d_S, p->s_pitch, p1_chirp(p), st))) return rc;
-        if ((rc = launch_rows(p, u0, n, d_out, out_pitch, st))) return rc;
+        if ((rc = launch_pass1(p, u0, n, p->d_S, p->s_pitch, p1_chirp(p), st, true))) return rc;
+        if ((rc = launch_rows(p, u0, n, d_out, out_pitch, st, (long)n * p->L <= PDL_ROWS_POINTS))) return rc;
     }
     return GBSP_OK;
 }
@@ -1058,7 +1087,8 @@ int p1b_dispatch(gbsp_batch_s* b, bool prepare, int sms, cudaStream_t st) {
         b->p1_grid = nb * sms;
         return GBSP_OK;
     }
-    return gbsp::p1_batch_launch(k, b->p1_grid, b->p1_smem, st, b->d_p1, b->d_p1_begin, b->n_fp32, b->d_queue);
+    return gbsp::p1_batch_launch(k, b->p1_grid, b->p1_smem, st, b->d_p1, b->d_p1_begin, b->n_fp32, b->d_queue,
+                                 b->n_mma > 0);
 }
 
 int batch_launch(gbsp_batch_s* b, cudaStream_t st) {
@@ -1074,7 +1104,7 @@ int batch_launch(gbsp_batch_s* b, cudaStream_t st) {
             const auto& k = b->classes[c];
             if ((rc = gbsp::rows_batch_launch(k.rb, k.pad, k.grid, k.smem, st, b->d_rows + k.begin,
                                               b->d_row_begin + k.begin + c, k.end - k.begin, b->d_queue + 2 + c,
-                                              b->d_err)))
+                                              c > 0, b->d_err)))
                 return rc;
         }
     }

@@ -207,7 +207,7 @@ std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_op
     std::vector<RadixPlan> out;
     for (const auto& rs : cands) {
         FFTDesc fd{};
-        if (build_fft_desc(Lp, rs, &fd, single ? smem_cap : 0) != GBSP_OK) continue;
+        if (build_fft_desc(Lp, rs, &fd, smem_cap) != GBSP_OK) continue;
         if (rows_smem_bytes(fd) > smem_cap) continue;
         const int rmax = *std::max_element(rs.begin(), rs.end());
         const int nt_hi = rmax > max_radix_for(1024) ? 512 : 1024;

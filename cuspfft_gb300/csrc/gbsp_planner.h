@@ -36,8 +36,7 @@ struct RadixPlan {
 };
 // Every (radix sequence, block size) for channel length Lp that fits in
 // smem_cap, cheapest first by rows_cost.  radix_opt (0-terminated, may be
-// null) and nt_opt (0 = automatic: 256 or 512) restrict the set; single: K = 1
-// (padded buffers allowed).
+// null) and nt_opt (0 = automatic: 256 or 512) restrict the set; single: K = 1.
 std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_opt, int nt_opt,
                                     bool direct, bool single, int rows_per_sm);
 

@@ -1,6 +1,6 @@
 // gbsp_rows_impl.cuh -- launch helpers shared by the translation units that
 // compile the multi-channel row kernels (gbsp_rows_multi.cu: clusters,
-// gbsp_rows_seq.cu: sequential channels).
+// gbsp_rows_seq*.cu: sequential channels).
 #pragma once
 #include "gbsp_launch.h"
 
@@ -25,9 +25,9 @@ inline cudaLaunchConfig_t config(const RowsKernel& k, unsigned grid, cudaStream_
     return cfg;
 }
 
-template <int NTMAX, int MODE>
+template <int NTMAX, int MODE, bool PAD = false>
 int capacity(const RowsKernel& k, int sms, int* cap) {
-    auto kern = k_bluestein_rows<NTMAX, MODE>;
+    auto kern = k_bluestein_rows<NTMAX, MODE, PAD>;
     if (int rc = allow_full_smem((const void*)kern)) return rc;
     if (MODE == ROW_CLUSTER) {
         cudaLaunchAttribute attr[1];
@@ -41,11 +41,10 @@ int capacity(const RowsKernel& k, int sms, int* cap) {
     return GBSP_OK;
 }
 
-template <int NTMAX, int MODE>
-int launch(const RowsKernel& k, int grid, cudaStream_t st, const RowsArgs& a, const FFTDesc& fd, int* err) {
-    cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = config(k, (unsigned)grid, st, attr);
-    GB_CUDA(cudaLaunchKernelEx(&cfg, k_bluestein_rows<NTMAX, MODE>, a, fd, err));
+template <int NTMAX, int MODE, bool PAD = false>
+int launch(const RowsKernel& k, int grid, cudaStream_t st, bool pdl, const RowsArgs& a, const FFTDesc& fd, int* err) {
+    GB_CUDA(launch_kernel(k_bluestein_rows<NTMAX, MODE, PAD>, grid, k.nt, k.smem, st, pdl,
+                          MODE == ROW_CLUSTER ? k.K : 1, a, fd, err));
     return GBSP_OK;
 }
 

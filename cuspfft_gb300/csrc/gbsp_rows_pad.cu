@@ -11,13 +11,13 @@ int rows_capacity_pad(const RowsKernel& k, int sms, int* cap) {
     return k.ntmax == 512 ? capacity<512, ROW_SINGLE, true>(k, sms, cap) : capacity<1024, ROW_SINGLE, true>(k, sms, cap);
 }
 
-int rows_launch_pad(const RowsKernel& k, int grid, cudaStream_t st, const RowsArgs& a, const FFTDesc& fd, int* err) {
+int rows_launch_pad(const RowsKernel& k, int grid, cudaStream_t st, bool pdl, const RowsArgs& a, const FFTDesc& fd, int* err) {
     using namespace rows_single;
     if (k.mode == ROW_DIRECT)
-        return k.ntmax == 512 ? launch<512, ROW_DIRECT, true>(k, grid, st, a, fd, err)
-                              : launch<1024, ROW_DIRECT, true>(k, grid, st, a, fd, err);
-    return k.ntmax == 512 ? launch<512, ROW_SINGLE, true>(k, grid, st, a, fd, err)
-                          : launch<1024, ROW_SINGLE, true>(k, grid, st, a, fd, err);
+        return k.ntmax == 512 ? launch<512, ROW_DIRECT, true>(k, grid, st, pdl, a, fd, err)
+                              : launch<1024, ROW_DIRECT, true>(k, grid, st, pdl, a, fd, err);
+    return k.ntmax == 512 ? launch<512, ROW_SINGLE, true>(k, grid, st, pdl, a, fd, err)
+                          : launch<1024, ROW_SINGLE, true>(k, grid, st, pdl, a, fd, err);
 }
 
 }  // namespace gbsp

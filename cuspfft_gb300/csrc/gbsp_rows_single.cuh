@@ -18,9 +18,8 @@ int capacity(const RowsKernel& k, int sms, int* cap) {
 }
 
 template <int NTMAX, int MODE, bool PAD>
-int launch(const RowsKernel& k, int grid, cudaStream_t st, const RowsArgs& a, const FFTDesc& fd, int* err) {
-    k_bluestein_rows<NTMAX, MODE, PAD><<<grid, k.nt, k.smem, st>>>(a, fd, err);
-    GB_CUDA(cudaGetLastError());
+int launch(const RowsKernel& k, int grid, cudaStream_t st, bool pdl, const RowsArgs& a, const FFTDesc& fd, int* err) {
+    GB_CUDA(launch_kernel(k_bluestein_rows<NTMAX, MODE, PAD>, grid, k.nt, k.smem, st, pdl, 1, a, fd, err));
     return GBSP_OK;
 }
 
