@@ -432,11 +432,9 @@ bool mma_choice(const gbsp_plan_s* p, const gbsp_options* o, const int* col_ptr)
 }
 
 // force_p1: 1-based pass-1 shape imposed by a batch (one shape for all its
-// matrices); 0 leaves the choice to the options.  batch_rows: Bluestein rows
-// of the whole batch (0: the plan runs alone).
+// matrices); 0 leaves the choice to the options.
 int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int* sparse_cols,
-               const gbsp_options* o_in, cudaStream_t st, int force_p1 = 0,
-               long batch_rows = 0) {
+               const gbsp_options* o_in, cudaStream_t st, int force_p1 = 0) {
     gbsp_options o = o_in ? *o_in : gbsp_options{};
     if (force_p1) o.pass1_shape = force_p1;
     GB_CUDA(cudaGetDevice(&p->device));
@@ -457,8 +455,7 @@ int plan_build(gbsp_plan_s* p, const int* col_ptr, const int* row_idx, const int
 
     // ---- lengths, channel split, radices and row block
     gbsp::ChannelSplit sp;
-    if ((rc = gbsp::split_channels(p->cols, batch_rows ? batch_rows : gbsp::launch_rows_of(p->rows, &o), &o, smem_cap,
-                                   &sp))) return rc;
+    if ((rc = gbsp::split_channels(p->cols, gbsp::launch_rows_of(p->rows, &o), &o, smem_cap, &sp))) return rc;
     p->L = sp.L;
     p->K = sp.K;
     p->Lp = sp.Lp;
@@ -1176,8 +1173,6 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
     o.rows_threads = 0;
     o.row_table_mode = 0;
     for (int& r : o.radix) r = 0;  // lengths differ across the batch: per-matrix radices
-    long all_rows = 0;
-    for (int i = 0; i < count; i++) all_rows += mats[i].rows / 2 + 1;
     b->plans.assign(count, nullptr);
     for (int i = 0; i < count && rc == GBSP_OK; i++) {
         gbsp_plan_s* p = new (std::nothrow) gbsp_plan_s();
@@ -1187,7 +1182,7 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
         p->nnz = mats[i].nnz;
         p->n_active = mats[i].n_active;
         b->plans[i] = p;
-        rc = plan_build(p, mats[i].col_ptr, mats[i].row_idx, mats[i].sparse_cols, &o, st, b->p1_shape, all_rows);
+        rc = plan_build(p, mats[i].col_ptr, mats[i].row_idx, mats[i].sparse_cols, &o, st, b->p1_shape);
     }
     if (rc) {
         free_batch(b);
@@ -1198,6 +1193,10 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
     // decreasing channel length inside a class.
     std::vector<int> per_sm(count, 0);
     std::vector<gbsp::RowBlock> rbs(count);
+    // (a matrix keeps the radices it has alone, so its spectrum keeps its
+    // bits; the block goes by the rows of the whole batch)
+    long all_rows = 0;
+    for (int i = 0; i < count; i++) all_rows += b->plans[i]->half_rows;
     for (int i = 0; i < count; i++) {
         const gbsp_plan_s* p = b->plans[i];
         if (p->K != 1 || p->rows_threads > 512) {
