@@ -28,7 +28,7 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompil
               f"-I{INCLUDE}", f"-I{CSRC}"]
 
 LIB_SOURCES = ["gbsp_rows_multi.cu", "gbsp_rows_seq.cu", "gbsp_rows_seq2.cu", "gbsp_rows_seq_pad.cu",
-               "gbsp_rows.cu", "gbsp_rows_pad.cu", "gbsp_rows_batch.cu",
+               "gbsp_rows.cu", "gbsp_rows_384.cu", "gbsp_rows_pad.cu", "gbsp_rows_batch.cu",
                "gbsp_rows_batch_pad.cu", "gbsp_pass1.cu", "gbsp_pass1_exact.cu", "gbsp_pass1_mma.cu",
                "gbsp_plan.cu", "gbsp_planner.cu", "gbsp_mlp.cu", "gbsp_host.cpp", "sparse_fft_api.cu"]
 CLI_SOURCES = ["cli_main.cpp"]

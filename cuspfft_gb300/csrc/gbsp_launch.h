@@ -89,7 +89,8 @@ int p1_mma_launch(int sms, size_t smem, cudaStream_t st, bool pdl, const P1MmaAr
 int p1_mma_batch_launch(int grid, size_t smem, cudaStream_t st, const P1MmaArgs* args, const long* item_begin,
                         int nmat, unsigned int* queue);
 
-// ---- Bluestein rows: mode ROW_*, compiled block bound ntmax (512 or 1024)
+// ---- Bluestein rows: mode ROW_*, compiled block bound ntmax (512 or 1024;
+// 384 for ROW_SINGLE without padding)
 struct RowsKernel {
     int mode, ntmax, K, nt;
     size_t smem;
@@ -98,6 +99,10 @@ struct RowsKernel {
 // CTAs (single channel, sequential channels) or clusters resident at once
 int rows_capacity(const RowsKernel& k, int sms, int* cap);
 int rows_launch(const RowsKernel& k, int grid, cudaStream_t st, bool pdl, const RowsArgs& a, const FFTDesc& fd, int* err);
+// ... ROW_SINGLE at 168 registers a thread (gbsp_rows_384.cu)
+int rows_capacity_384(const RowsKernel& k, int sms, int* cap);
+int rows_launch_384(const RowsKernel& k, int grid, cudaStream_t st, bool pdl, const RowsArgs& a, const FFTDesc& fd,
+                    int* err);
 // ... with a padded row buffer (gbsp_rows_pad.cu)
 int rows_capacity_pad(const RowsKernel& k, int sms, int* cap);
 int rows_launch_pad(const RowsKernel& k, int grid, cudaStream_t st, bool pdl, const RowsArgs& a, const FFTDesc& fd, int* err);

@@ -360,7 +360,7 @@ int rows_prepare(gbsp_plan_s* p, int sms) {
     }
     p->rows_block = p->rows_threads;
     if (p->K == 1) {
-        const RowBlock rb = choose_row_block(p->fd, p->rows_threads, p->u_tile / sms);
+        const RowBlock rb = choose_row_block(p->fd, p->rows_threads, p->u_tile / sms, p->direct != 0);
         p->rows_block = rb.nt;
         p->rows_ntmax = rb.ntmax;
     }
@@ -1203,7 +1203,9 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
             b->separate.push_back(i);
             continue;
         }
-        rbs[i] = gbsp::choose_row_block(p->fd, p->rows_threads, (int)std::min<long>(all_rows / sms, 1 << 20));
+        rbs[i] = gbsp::choose_row_block(p->fd, p->rows_threads, (int)std::min<long>(all_rows / sms, 1 << 20),
+                                        p->direct != 0);
+        rbs[i].ntmax = std::max(rbs[i].ntmax, 512);  // the batched kernel has no 384-thread instance
         if (gbsp::rows_batch_blocks_per_sm(rbs[i], p->fd.sh < 31, rows_smem_bytes(p->fd), &per_sm[i]) != GBSP_OK || per_sm[i] < 1) {
             free_batch(b);
             return set_error(GBSP_ERR_UNSUPPORTED, "gbsp_batch_create: batched row kernel does not fit");
@@ -1430,7 +1432,9 @@ extern "C" int gbsp_execute_to_host(gbsp_plan_t p, void* h_out, size_t out_pitch
     // about as fast as the one before it copies out.  Ramp tiles are
     // multiples of 256 rows (the largest pass-1 row block), so a tile size
     // that is one too starts every tile where the single launch starts a
-    // row block, with the same bits.
+    // row block, with the same bits where that launch runs the FP32 pass 1 too
+    // (tiles below MMA_MIN_ROWS rows stay on it; they agree to rounding with a
+    // launch on the tensor cores).
     int n_ramp = std::min(tile, 256);
     for (int u0 = 0, n = 0; u0 < p->half_rows && rc == GBSP_OK; u0 += n, t++) {
         n = std::min(n_ramp, p->half_rows - u0);

@@ -179,10 +179,34 @@ double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct, bo
 // radix 16 spills there (2048 points [16, 16, 8] 254 -> 261 us).
 constexpr int BLOCK32_POINTS = 700, BLOCK64_POINTS = 3000, BLOCK128_POINTS = 7000, REGS64_RADIX = 15;
 
-RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm) {
+//
+// Long rows (512 threads, one block an SM): a stage of nb butterflies runs
+// rounds of the block, each as long as its warps need to issue it or, with
+// few, as one butterfly takes alone (about 2.2 warps' worth per scheduler).
+// Where 352 threads shorten that sum by a tenth they are taken, at 168
+// registers a thread (no spills).  GB300, 6007 rows, 512 -> 352 threads: 16464
+// points [28, 28, 21] 474 -> 428 us, 18816 [32, 28, 21] 510 -> 486, 21504
+// [32, 32, 21] 564 -> 534, 21609 [21, 21, 7, 7] 619 -> 606, 15625 [25, 25, 25]
+// 452 both.  Nearer 1 it may lose: 15750 [2, 25, 21, 15] (0.90) 544 -> 553.
+static double round_cost(const FFTDesc& fd, int nt) {
+    constexpr double kAlone = 2.2;
+    double cost = 0.0;
+    for (int s = 0; s < fd.nst; s++) {
+        const int nb = fd.Lp / fd.R[s], rem = nb % nt;
+        const double rounds = (nb / nt) * std::max(nt / 128.0, kAlone) + (rem ? std::max(rem / 128.0, kAlone) : 0.0);
+        cost += (s == fd.nst - 1 ? 1.0 : 2.0) * fd.R[s] * rounds;
+    }
+    return cost;
+}
+
+RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm, bool direct) {
     int rmax = 0;
     for (int s = 0; s < fd.nst; s++) rmax = std::max(rmax, fd.R[s]);
     RowBlock b{nt, (rmax > max_radix_for(1024) || nt <= 512) ? 512 : 1024};
+    if (nt == 512 && !direct && fd.sh == 31 && rows_smem_bytes(fd) > kSmemPerSM / 2) {
+        if (round_cost(fd, 352) < 0.9 * round_cost(fd, 512)) b = RowBlock{352, 384};
+        return b;
+    }
     if (nt != 256 || fd.Lp > BLOCK128_POINTS) return b;
     b.nt = fd.Lp <= BLOCK32_POINTS ? 32 : fd.Lp <= BLOCK64_POINTS ? 64 : 128;
     // 512 threads an SM at 128 registers: with fewer rows, wider blocks
@@ -220,7 +244,7 @@ std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_op
             rp.fd = fd;
             rp.nt = nt;
             // at the block it is launched with
-            const int block = single ? choose_row_block(fd, nt, rows_per_sm).nt : nt;
+            const int block = single && nt == 256 ? choose_row_block(fd, nt, rows_per_sm, direct).nt : nt;
             rp.cost = rows_cost(fd, block, rows_smem_bytes(fd), direct);
             out.push_back(rp);
         }

@@ -22,12 +22,12 @@ int max_radix_for(int nt_max);  // largest radix a block of at most nt_max threa
 double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct = false, bool feature = false);
 
 // The block a single-channel row planned for nt threads is launched with, and
-// the compiled block bound of its kernel (512: 128 registers a thread, 1024:
-// 64).  rows_per_sm: rows there are for each SM.
+// the compiled block bound of its kernel (384: 168 registers a thread, 512:
+// 128, 1024: 64).  rows_per_sm: rows there are for each SM.
 struct RowBlock {
     int nt, ntmax;
 };
-RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm);
+RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm, bool direct);
 
 struct RadixPlan {
     FFTDesc fd{};

@@ -7,6 +7,7 @@
 namespace gbsp {
 int rows_capacity(const RowsKernel& k, int sms, int* cap) {
     *cap = 0;
+    if (k.ntmax == 384) return rows_capacity_384(k, sms, cap);
     if (k.pad && k.K == 1) return rows_capacity_pad(k, sms, cap);
     if (k.mode == ROW_DIRECT)
         return k.ntmax == 512 ? rows_single::capacity<512, ROW_DIRECT, false>(k, sms, cap)
@@ -17,6 +18,7 @@ int rows_capacity(const RowsKernel& k, int sms, int* cap) {
 }
 
 int rows_launch(const RowsKernel& k, int grid, cudaStream_t st, bool pdl, const RowsArgs& a, const FFTDesc& fd, int* err) {
+    if (k.ntmax == 384) return rows_launch_384(k, grid, st, pdl, a, fd, err);
     if (k.pad && k.K == 1) return rows_launch_pad(k, grid, st, pdl, a, fd, err);
     if (k.mode == ROW_DIRECT)
         return k.ntmax == 512 ? rows_single::launch<512, ROW_DIRECT, false>(k, grid, st, pdl, a, fd, err)

@@ -97,7 +97,8 @@ typedef struct {
                               in [64, 1024] (at most 512 when a radix exceeds 16).
                               Rows of up to 7000 points planned for 256 threads are
                               launched in blocks of 32, 64 or 128 when there are
-                              enough of them                                              */
+                              enough of them, long ones planned for 512 in 352
+                              where that divides their stages better                      */
     int row_table_mode;    /* pass-1 twiddle table: 0 = auto, 1 = full circle,
                               2 = half circle, 3 = two-level (W^p = hi[p/256]*lo[p%256],
                               any row count)                                              */

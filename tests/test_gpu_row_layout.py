@@ -2,7 +2,8 @@
 
 Short rows run in blocks of 32, 64 or 128 threads when there are enough of
 them (edges at 700, 3000 and 7000 points), on the 64- or 128-register kernels;
-rows whose last radix is a power of two use a padded row buffer.  The rel-L2
+long ones planned for 512 threads in 352 where that divides their stages
+better; rows whose last radix is a power of two use a padded row buffer.  The rel-L2
 bar is 1e-6: an FP32 FFT of up to five stages and its inverse round each value
 about 30 times at 6e-8, 3.3e-7 when independent, three times that at worst here.
 """
@@ -41,6 +42,15 @@ def check(coo, **kw):
 @pytest.mark.parametrize("rows", [311, 2500, 12000])
 def test_block_widths(cuda, rows, cols):
     coo = synthetic.uniform_matrix(rows, cols, 3 * max(rows, cols), seed=cols)
+    check(coo, length_policy=gb.GBSP_LEN_7SMOOTH)
+
+
+# long rows: three and four stages that 352 threads divide better than 512
+# (7813, 8231, 9407, 10805), and some that stay
+@pytest.mark.parametrize("cols", [7499, 7813, 7874, 8231, 8959, 9407, 10805, 11003])
+@pytest.mark.parametrize("rows", [303, 1201])
+def test_long_row_blocks(cuda, rows, cols):
+    coo = synthetic.uniform_matrix(rows, cols, 3 * cols, seed=cols)
     check(coo, length_policy=gb.GBSP_LEN_7SMOOTH)
 
 
