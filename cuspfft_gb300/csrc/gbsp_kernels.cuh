@@ -438,13 +438,11 @@ __global__ void __launch_bounds__(P1_THREADS, 1) k_twiddle_sum(P1Args a) {
 // each matrix, item_begin[nmat] = total) handed out by a device work queue,
 // one item per grab.  Items are grabbed in increasing order, so a CTA moves
 // forward through the matrices and reloads the twiddle table only when it
-// enters a new one.  *queue must be 0 at launch.  late: the kernel before it in
-// the stream is independent (the tensor-core part of pass 1), so only the
-// kernel's end waits for it.
+// enters a new one.  *queue must be 0 at launch.
 template <typename IDX, int TAB, bool BIG, int KU, bool EXACT>
 __global__ void __launch_bounds__(P1_THREADS, 1)
 k_twiddle_sum_batch(const P1Args* __restrict__ args, const long* __restrict__ item_begin, int nmat,
-                    unsigned long long* queue, int late) {
+                    unsigned long long* queue) {
     extern __shared__ float4 smem_raw[];
     __shared__ P1Shared sh;
     __shared__ P1Args cur;
@@ -454,7 +452,7 @@ k_twiddle_sum_batch(const P1Args* __restrict__ args, const long* __restrict__ it
     int loaded = -1;
     pdl_trigger();
     if (threadIdx.x == 0) { sh.next_task = 0; s_m = 0; }
-    if (!late) pdl_wait();
+    pdl_wait();
     __syncthreads();
     const long total = item_begin[nmat];
     for (;;) {
@@ -482,7 +480,6 @@ k_twiddle_sum_batch(const P1Args* __restrict__ args, const long* __restrict__ it
         float2* tab = reinterpret_cast<float2*>(info_all + P1_WARPS * 32);
         p1_item<IDX, TAB, BIG, KU, EXACT>(cur, it - item_begin[m], stage, info_all, tab, sh);
     }
-    if (late && blockIdx.x == 0) pdl_wait();
 }
 
 // ---------------------------------------------------------------------------
@@ -970,10 +967,7 @@ __global__ void __launch_bounds__(NTMAX, 1) k_bluestein_rows(RowsArgs a, FFTDesc
 // matrices in order and reloads the matrix's descriptor and stage twiddles
 // only when it moves to the next one.  Shared memory holds the largest
 // matrix's row buffer plus its stage twiddles (the twiddles of each matrix
-// sit right after its own row buffer).  *queue must be 0 at launch.  late: the
-// kernel before it in the stream is the rows of another class, which started
-// after pass 1 was complete; only the kernel's end waits for it, so that its
-// blocks fill the SMs the other class leaves.
+// sit right after its own row buffer).  *queue must be 0 at launch.
 struct RowsBatch {
     RowsArgs a;
     FFTDesc fd;
@@ -982,7 +976,7 @@ struct RowsBatch {
 template <int NTMAX, bool PAD>
 __global__ void __launch_bounds__(NTMAX, 1)
 k_bluestein_rows_batch(const RowsBatch* __restrict__ descs, const long* __restrict__ row_begin, int nmat,
-                       unsigned long long* queue, int late, int* err) {
+                       unsigned long long* queue, int* err) {
     extern __shared__ float4 smem_raw[];
     __shared__ uint64_t in_bar;
     __shared__ RowsBatch cur;
@@ -1000,8 +994,7 @@ k_bluestein_rows_batch(const RowsBatch* __restrict__ descs, const long* __restri
     int err_bits = 0;
     int loaded = -1;
     const long total = row_begin[nmat];
-    // the successor may start once pass 1 is known to be complete
-    if (!late) pdl_wait();
+    pdl_wait();
     pdl_trigger();
     __syncthreads();
     for (;;) {
@@ -1028,7 +1021,6 @@ k_bluestein_rows_batch(const RowsBatch* __restrict__ descs, const long* __restri
         bluestein_row<MAXR, ROW_SINGLE, PAD, 2>(cur.a, cur.fd, (int)(t - row_begin[m]), 0, buf, twr, zsrc, &in_bar,
                                                 parity, err_bits);
     }
-    if (late && blockIdx.x == 0) pdl_wait();
     if (err_bits) atomicOr(err, err_bits);
     if (err_bits & ERR_TIMEOUT) mbar_wait_bounded(&in_bar, parity ^ 1u);
 }

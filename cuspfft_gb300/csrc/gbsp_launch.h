@@ -81,7 +81,7 @@ int p1_blocks_per_sm(const P1Kernel& k, size_t smem, int* nb);
 int p1_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, bool pdl, const P1Args& a);
 int p1_batch_blocks_per_sm(const P1Kernel& k, size_t smem, int* nb);
 int p1_batch_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, const P1Args* args,
-                    const long* item_begin, int nmat, unsigned long long* queue, bool late);
+                    const long* item_begin, int nmat, unsigned long long* queue);
 
 // ---- pass 1 on the tensor cores (gbsp_pass1_mma.cu), one CTA per SM
 int p1_mma_prepare(size_t smem, bool batch);  // raises the limit, checks that it fits
@@ -110,9 +110,9 @@ int rows_launch_pad(const RowsKernel& k, int grid, cudaStream_t st, bool pdl, co
 int rows_batch_blocks_per_sm(const RowBlock& rb, bool pad, size_t smem, int* nb);
 int rows_batch_blocks_per_sm_pad(const RowBlock& rb, size_t smem, int* nb);
 int rows_batch_launch_pad(const RowBlock& rb, int grid, size_t smem, cudaStream_t st, const RowsBatch* descs,
-                          const long* row_begin, int nmat, unsigned long long* queue, bool late, int* err);
+                          const long* row_begin, int nmat, unsigned long long* queue, bool pdl, int* err);
 int rows_batch_launch(const RowBlock& rb, bool pad, int grid, size_t smem, cudaStream_t st, const RowsBatch* descs,
-                      const long* row_begin, int nmat, unsigned long long* queue, bool late, int* err);
+                      const long* row_begin, int nmat, unsigned long long* queue, bool pdl, int* err);
 // the multi-channel modes (clusters: gbsp_rows_multi.cu, sequential
 // channels: gbsp_rows_seq.cu); rows_capacity / rows_launch forward to these
 int rows_capacity_multi(const RowsKernel& k, int sms, int* cap);

@@ -20,9 +20,9 @@ int p1_batch_blocks_per_sm(const P1Kernel& k, size_t smem, int* nb) {
 }
 
 int p1_batch_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, const P1Args* args,
-                    const long* item_begin, int nmat, unsigned long long* queue, bool late) {
-    return k.exact ? Pass1Set<true>::batch_launch(k, grid, smem, st, args, item_begin, nmat, queue, late)
-                   : Pass1Set<false>::batch_launch(k, grid, smem, st, args, item_begin, nmat, queue, late);
+                    const long* item_begin, int nmat, unsigned long long* queue) {
+    return k.exact ? Pass1Set<true>::batch_launch(k, grid, smem, st, args, item_begin, nmat, queue)
+                   : Pass1Set<false>::batch_launch(k, grid, smem, st, args, item_begin, nmat, queue);
 }
 
 }  // namespace gbsp

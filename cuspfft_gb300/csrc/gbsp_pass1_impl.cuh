@@ -30,9 +30,9 @@ struct P1Ops {
         return GBSP_OK;
     }
     static int batch_launch(int grid, size_t smem, cudaStream_t st, const P1Args* args, const long* item_begin,
-                            int nmat, unsigned long long* queue, bool late) {
-        GB_CUDA(launch_kernel(k_twiddle_sum_batch<IDX, TAB, BIG, KU, EXACT>, grid, P1_THREADS, smem, st, late, 1, args,
-                              item_begin, nmat, queue, (int)late));
+                            int nmat, unsigned long long* queue) {
+        GB_CUDA(launch_kernel(k_twiddle_sum_batch<IDX, TAB, BIG, KU, EXACT>, grid, P1_THREADS, smem, st, false, 1, args,
+                              item_begin, nmat, queue));
         return GBSP_OK;
     }
 };
@@ -70,9 +70,9 @@ struct Pass1Set {
         return with_p1<EXACT>(k, [&](auto ops) { return decltype(ops)::batch_blocks(smem, nb); });
     }
     static int batch_launch(const P1Kernel& k, int grid, size_t smem, cudaStream_t st, const P1Args* args,
-                            const long* item_begin, int nmat, unsigned long long* queue, bool late) {
+                            const long* item_begin, int nmat, unsigned long long* queue) {
         return with_p1<EXACT>(k, [&](auto ops) {
-            return decltype(ops)::batch_launch(grid, smem, st, args, item_begin, nmat, queue, late);
+            return decltype(ops)::batch_launch(grid, smem, st, args, item_begin, nmat, queue);
         });
     }
 };

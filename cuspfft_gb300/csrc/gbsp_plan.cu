@@ -1051,6 +1051,10 @@ struct gbsp_batch_s {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     std::vector<void*> allocs;
+    // side streams and events for launches that may overlap (batch_overlap)
+    cudaEvent_t fork = nullptr;
+    std::vector<cudaStream_t> side;
+    std::vector<cudaEvent_t> join;
 };
 
 namespace {
@@ -1061,6 +1065,9 @@ void free_batch(gbsp_batch_s* b) {
     if (b->graph) cudaGraphDestroy(b->graph);
     for (auto* p : b->plans) free_plan(p);
     for (void* a : b->allocs) cudaFree(a);
+    if (b->fork) cudaEventDestroy(b->fork);
+    for (auto e : b->join) cudaEventDestroy(e);
+    for (auto s : b->side) cudaStreamDestroy(s);
     delete b;
 }
 
@@ -1084,26 +1091,66 @@ int p1b_dispatch(gbsp_batch_s* b, bool prepare, int sms, cudaStream_t st) {
         b->p1_grid = nb * sms;
         return GBSP_OK;
     }
-    return gbsp::p1_batch_launch(k, b->p1_grid, b->p1_smem, st, b->d_p1, b->d_p1_begin, b->n_fp32, b->d_queue,
-                                 b->n_mma > 0);
+    return gbsp::p1_batch_launch(k, b->p1_grid, b->p1_smem, st, b->d_p1, b->d_p1_begin, b->n_fp32, b->d_queue);
+}
+
+// Side streams for n launches at once: at most 7, as a device runs eight
+// queues by default; more launches take turns on them.
+constexpr int MAX_SIDE_STREAMS = 7;
+int batch_side_streams(gbsp_batch_s* b, int n) {
+    n = std::min(n - 1, MAX_SIDE_STREAMS);
+    if (n < 1) return GBSP_OK;
+    GB_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+    for (int i = 0; i < n; i++) {
+        cudaStream_t s = nullptr;
+        GB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        b->side.push_back(s);
+        cudaEvent_t e = nullptr;
+        GB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        b->join.push_back(e);
+    }
+    return GBSP_OK;
+}
+
+// n launches that do not depend on one another, launch(i, stream): the first
+// on st, the others on side streams that start after all st holds and that st
+// waits for.  Each so has a full dependency on what was launched before
+// (launched programmatically one after another, the later ones would read S
+// without a wait of their own); in a capture they become parallel nodes.
+template <typename F>
+int batch_overlap(gbsp_batch_s* b, cudaStream_t st, int n, F&& launch) {
+    const int ns = std::min(n - 1, (int)b->side.size());
+    if (ns > 0) GB_CUDA(cudaEventRecord(b->fork, st));
+    for (int i = 0; i < ns; i++) GB_CUDA(cudaStreamWaitEvent(b->side[i], b->fork, 0));
+    int rc = GBSP_OK;
+    for (int i = 0; i < n && rc == GBSP_OK; i++) rc = launch(i, i == 0 ? st : b->side[(i - 1) % ns]);
+    for (int i = 0; i < ns; i++) {  // after an error too
+        GB_CUDA(cudaEventRecord(b->join[i], b->side[i]));
+        GB_CUDA(cudaStreamWaitEvent(st, b->join[i], 0));
+    }
+    return rc;
 }
 
 int batch_launch(gbsp_batch_s* b, cudaStream_t st) {
     if (!b->order.empty()) {
         GB_CUDA(cudaMemsetAsync(b->d_queue, 0, (2 + b->classes.size()) * sizeof(unsigned long long), st));
-        int rc = GBSP_OK;
-        if (b->n_mma > 0 &&
-            (rc = gbsp::p1_mma_batch_launch(b->mma_grid, b->mma_smem, st, b->d_mma, b->d_mma_begin, b->n_mma,
-                                            reinterpret_cast<unsigned int*>(b->d_queue + 1))))
-            return rc;
-        if (b->n_fp32 > 0 && (rc = p1b_dispatch(b, false, 0, st))) return rc;
-        for (size_t c = 0; c < b->classes.size(); c++) {
+        // pass 1: the tensor-core and the FP32 matrices
+        const bool both = b->n_mma > 0 && b->n_fp32 > 0;
+        int rc = batch_overlap(b, st, both ? 2 : 1, [&](int i, cudaStream_t s) {
+            if (i == 0 && b->n_mma > 0)
+                return gbsp::p1_mma_batch_launch(b->mma_grid, b->mma_smem, s, b->d_mma, b->d_mma_begin, b->n_mma,
+                                                 reinterpret_cast<unsigned int*>(b->d_queue + 1));
+            return p1b_dispatch(b, false, 0, s);
+        });
+        if (rc) return rc;
+        // the rows, class by class; the first may start while pass 1 ends
+        rc = batch_overlap(b, st, (int)b->classes.size(), [&](int c, cudaStream_t s) {
             const auto& k = b->classes[c];
-            if ((rc = gbsp::rows_batch_launch(k.rb, k.pad, k.grid, k.smem, st, b->d_rows + k.begin,
-                                              b->d_row_begin + k.begin + c, k.end - k.begin, b->d_queue + 2 + c,
-                                              c > 0, b->d_err)))
-                return rc;
-        }
+            return gbsp::rows_batch_launch(k.rb, k.pad, k.grid, k.smem, s, b->d_rows + k.begin,
+                                           b->d_row_begin + k.begin + c, k.end - k.begin, b->d_queue + 2 + c,
+                                           c == 0 && !both, b->d_err);
+        });
+        if (rc) return rc;
     }
     for (int m : b->separate) {
         int rc = gbsp_execute(b->plans[m], b->outs[m], b->pitches[m], st);
@@ -1278,7 +1325,8 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
         }
     }
     if ((rc = batch_alloc(b, (void**)&b->d_queue, (2 + ncls) * sizeof(unsigned long long))) ||
-        (rc = batch_alloc(b, (void**)&b->d_err, sizeof(int)))) {
+        (rc = batch_alloc(b, (void**)&b->d_err, sizeof(int))) ||
+        (rc = batch_side_streams(b, std::max(ncls, b->n_mma > 0 && b->n_fp32 > 0 ? 2 : 1)))) {
         free_batch(b);
         return rc;
     }

@@ -8,9 +8,9 @@ int rows_batch_blocks_per_sm(const RowBlock& rb, bool pad, size_t smem, int* nb)
 }
 
 int rows_batch_launch(const RowBlock& rb, bool pad, int grid, size_t smem, cudaStream_t st, const RowsBatch* descs,
-                      const long* row_begin, int nmat, unsigned long long* queue, bool late, int* err) {
-    return pad ? rows_batch_launch_pad(rb, grid, smem, st, descs, row_begin, nmat, queue, late, err)
-               : rows_batch::launch<false>(rb, grid, smem, st, descs, row_begin, nmat, queue, late, err);
+                      const long* row_begin, int nmat, unsigned long long* queue, bool pdl, int* err) {
+    return pad ? rows_batch_launch_pad(rb, grid, smem, st, descs, row_begin, nmat, queue, pdl, err)
+               : rows_batch::launch<false>(rb, grid, smem, st, descs, row_begin, nmat, queue, pdl, err);
 }
 
 }  // namespace gbsp

@@ -21,9 +21,9 @@ int blocks_per_sm(const RowBlock& rb, size_t smem, int* nb) {
 
 template <bool PAD>
 int launch(const RowBlock& rb, int grid, size_t smem, cudaStream_t st, const RowsBatch* descs, const long* row_begin,
-           int nmat, unsigned long long* queue, bool late, int* err) {
+           int nmat, unsigned long long* queue, bool pdl, int* err) {
     GB_CUDA(launch_kernel(rb.ntmax == 512 ? k_bluestein_rows_batch<512, PAD> : k_bluestein_rows_batch<1024, PAD>, grid,
-                          rb.nt, smem, st, true, 1, descs, row_begin, nmat, queue, (int)late, err));
+                          rb.nt, smem, st, pdl, 1, descs, row_begin, nmat, queue, err));
     return GBSP_OK;
 }
 

@@ -8,8 +8,8 @@ int rows_batch_blocks_per_sm_pad(const RowBlock& rb, size_t smem, int* nb) {
 }
 
 int rows_batch_launch_pad(const RowBlock& rb, int grid, size_t smem, cudaStream_t st, const RowsBatch* descs,
-                          const long* row_begin, int nmat, unsigned long long* queue, bool late, int* err) {
-    return rows_batch::launch<true>(rb, grid, smem, st, descs, row_begin, nmat, queue, late, err);
+                          const long* row_begin, int nmat, unsigned long long* queue, bool pdl, int* err) {
+    return rows_batch::launch<true>(rb, grid, smem, st, descs, row_begin, nmat, queue, pdl, err);
 }
 
 }  // namespace gbsp
