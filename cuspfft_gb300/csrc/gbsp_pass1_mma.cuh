@@ -544,6 +544,15 @@ k_twiddle_mma(P1MmaArgs one, const P1MmaArgs* __restrict__ args, const long* __r
             items++;
             cur = nxt;
         }
+        // No copy may be in flight when the CTA ends.  The warps that use a
+        // chunk wait for it, unless a wait gave up before.  (Before the end
+        // mark, which moves its slot's barrier on by one phase more.)
+        if (lane == 0) {
+            int alone = 0;
+            for (int k = max(0, n - MM_DESCS); k < n; k++)
+                mm_wait(&sh.desc_full[k % MM_DESCS], (k / MM_DESCS) & 1, &alone);
+        }
+        __syncwarp();
         if (ok && n >= MM_DESCS) ok = mm_wait_warp(&sh.desc_empty[n % MM_DESCS], (n / MM_DESCS - 1) & 1, dead);
         if (ok && lane == 0) {
             sh.desc[n % MM_DESCS].flags = MM_END;
