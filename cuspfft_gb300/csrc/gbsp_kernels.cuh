@@ -534,36 +534,34 @@ struct RowsArgs {
 };
 
 // The fold of a row longer than its channel q: slot n gets
-// sum_j W_L^{q (n + j*Lp)} * x[n + j*Lp] over at most NS sections; with
-// W_L^{q (n + j*Lp)} = W_L^{q n} * W_K^{q j} (pre[n] and pre[j*Lp]) one table
-// entry per slot instead of one per value, and none for channel 0 (PRE false).
+// sum_j W_L^{q (n + j*Lp)} * x[n + j*Lp] over at most NS sections, each value
+// times its own table entry pre[n + j*Lp] (one rounded factor; the product
+// W_L^{q n} * W_K^{q j} of two saves loads and adds a rounding), none for
+// channel 0, whose entries are 1 (PRE false).
 // U slots a pass, all their loads (L2) issued before any product: one slot a
 // pass waited out the L2 latency Lp / nt times per channel, 46 % of the row
 // kernel on 40421 columns (three channels of 27000, two sections).
 template <bool PRE, bool PAD, int NS, int U>
 __device__ __forceinline__ void fold_sections(float2* __restrict__ buf, const float2* __restrict__ x,
                                               const float2* __restrict__ pre, int cols, int Lp, int sh, int tid, int nt) {
-    float2 wk[NS];
-#pragma unroll
-    for (int j = 1; j < NS; j++) wk[j] = (PRE && j * Lp < cols) ? __ldg(pre + j * Lp) : make_float2(1.f, 0.f);
     for (int n0 = tid; n0 < Lp; n0 += U * nt) {
-        float2 xv[U][NS], pv[U];
+        float2 xv[U][NS], pv[U][NS];
 #pragma unroll
         for (int w = 0; w < U; w++) {
             const int n = n0 + w * nt;
 #pragma unroll
             for (int j = 0; j < NS; j++) {
                 const int c = n + j * Lp;
-                xv[w][j] = (n < Lp && c < cols) ? __ldcg(x + c) : make_float2(0.f, 0.f);
+                const bool ok = n < Lp && c < cols;
+                xv[w][j] = ok ? __ldcg(x + c) : make_float2(0.f, 0.f);
+                if (PRE) pv[w][j] = ok ? __ldg(pre + c) : make_float2(0.f, 0.f);
             }
-            if (PRE) pv[w] = n < Lp ? __ldg(pre + n) : make_float2(0.f, 0.f);
         }
 #pragma unroll
         for (int w = 0; w < U; w++) {
-            float2 acc = xv[w][0];
+            float2 acc = PRE ? cmul(xv[w][0], pv[w][0]) : xv[w][0];
 #pragma unroll
-            for (int j = 1; j < NS; j++) acc = cadd(acc, PRE ? cmul(xv[w][j], wk[j]) : xv[w][j]);
-            if (PRE) acc = cmul(acc, pv[w]);
+            for (int j = 1; j < NS; j++) acc = cadd(acc, PRE ? cmul(xv[w][j], pv[w][j]) : xv[w][j]);
             if (n0 + w * nt < Lp) buf[padded<PAD>(n0 + w * nt, sh)] = acc;
         }
     }
