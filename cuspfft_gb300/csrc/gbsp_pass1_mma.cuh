@@ -13,12 +13,17 @@
 // w = h + m + l: h to 2^-7, m to 2^-18, l the rest (all times 64, so that l
 // keeps its bits).  The h*h products are multiples of 2^-14, so their FP32
 // accumulation in TMEM, whose rounding is not to nearest, is exact while a
-// partial sum stays below 1024: columns of more nonzeros (MM_MAX_DEGREE) take
-// the FP32 kernel.  The products h*m, m*h, m*m, h*l, l*h go to a second
-// accumulator, 2^-8 as large, whose rounding does not matter (m*l and l*l are
-// below 2^-26).  What is left is the rounding of the two table entries: on
-// columns of 2 to 1000 nonzeros the sums are 2-4e-8 (relative L2) from FP64,
-// where FP32 sums of recurrence twiddles are 0.9-1.3e-7.
+// partial sum stays below 1024.  A rounded factor is at most 1 + 2^-7.5 long,
+// so that holds for any sum of up to 1012 nonzeros; columns of more than 1024
+// (MM_MAX_DEGREE) take the FP32 kernel, and between the two a sum past 1024,
+// which has 2^-13 as its own FP32 step, is cut to that step in the last one or
+// two K-steps (at most 6e-8 of it each).  The products h*m, m*h, m*m, h*l, l*h
+// go to a second accumulator, 2^-8 as large on random rows and at most 7 where
+// all of a column's factors are rounded the same way, which its rounding
+// shifts by 8e-8 of the sum at worst (m*l and l*l are below 2^-26 each).  What
+// is left is the rounding of the two table entries: on columns of 2 to 1000
+// nonzeros the sums are 2-4e-8 (relative L2) from FP64, where FP32 sums of
+// recurrence twiddles are 0.9-1.3e-7.
 //
 // A row's split depends on its tile only through u0 mod 128, so tiles that
 // start at a multiple of 128 rows give the same bits as one tile.
@@ -67,7 +72,7 @@ constexpr int MM_A_BYTES = MM_ROWS * 32;       // one part of A, one K-step
 constexpr int MM_B_BYTES = 2 * MM_MAXD * 32;   // one part of B, one K-step
 constexpr int MM_KSTEP_BYTES = 3 * (MM_A_BYTES + MM_B_BYTES);
 constexpr int MM_STAGE_BYTES = MM_KSTEPS * MM_KSTEP_BYTES;
-constexpr int MM_MAX_DEGREE = 1024;          // nonzeros of a column up to which the h*h sums are exact
+constexpr int MM_MAX_DEGREE = 1024;          // nonzeros of a column (h*h sums exact up to 1012, see above)
 constexpr uint32_t MM_PAD = 0xffffffffu;     // no fraction of rows < 2^31
 constexpr float MM_SCALE = 64.f;             // table entries in shared memory
 constexpr float MM_UNSCALE = 1.f / (MM_SCALE * MM_SCALE);

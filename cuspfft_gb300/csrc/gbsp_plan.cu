@@ -422,7 +422,8 @@ int learned_choice(const gbsp_plan_s* p, const int* col_ptr, size_t smem_cap, gb
 
 // Whether the tensor-core kernel runs pass 1 of a plan's large tiles.  Not in
 // the exact-phase mode (no products of twiddles) nor with an explicit Kahan
-// degree (a property of the FP32 sums), nor with columns past its exact range.
+// degree (a property of the FP32 sums), nor with columns past its accumulators'
+// range.
 bool mma_choice(const gbsp_plan_s* p, const gbsp_options* o, const int* col_ptr) {
     if (o->exact_phases != 0 || o->kahan_min_degree != 0 || p->mma_tab < 0) return false;
     if (p->u_tile < MMA_MIN_ROWS || (long long)p->u_tile * p->nnz < MMA_MIN_ROWS_PER_COL * p->cols) return false;

@@ -1,0 +1,45 @@
+"""The tensor-core pass 1 at the ends of its range.
+
+Degree limit.  At u = 0 all of a column's terms are 1, a product of W^{-64 r}
+and W^{64 r}, each a rounded table entry split into h (step 2^-7), m and l.
+The worst columns are the rows whose h is longest: the h*h sum then runs ahead
+of the true one, past 1024 at 1024 nonzeros, and the second accumulator holds a
+like amount of the other sign.  Against the sum of the rounded entries'
+products, in FP64: the first accumulator loses at most two steps of 2^-14 past
+1024 (1.2e-7 of the sum), the second half a step of its size per MMA, five in
+each of 128 K-steps, 8.4e-5 in all while it grows to 7 (8e-8), and the result
+is rounded once (6e-8): 2.6e-7, held to 3e-7.
+"""
+import numpy as np
+import pytest
+
+import cuspfft_gb300 as gb
+
+pytestmark = pytest.mark.gpu
+
+
+def sums(coo, us, **kw):
+    import torch
+    n = coo.rows // 2 + 1
+    with gb.Plan(coo, **kw) as p:
+        s = torch.empty((n, (coo.cols + 1) // 2 * 2), dtype=torch.complex64, device="cuda")
+        p.column_sums(0, n, s)
+        torch.cuda.synchronize()
+        assert p.error_flags() == 0
+        return s[torch.as_tensor(us, device="cuda"), :coo.cols].cpu().numpy().astype(np.complex128)
+
+
+@pytest.mark.parametrize("rows", [5003, 8219, 9001, 12007])
+def test_longest_factors_at_the_degree_limit(cuda, rows):
+    r = np.arange(rows, dtype=np.int64)
+    w = np.exp(-2j * np.pi * (64 * r % rows) / rows).astype(np.complex64).astype(np.complex128)
+    h = np.round(w.real * 128) ** 2 + np.round(w.imag * 128) ** 2
+    order = np.argsort(-h, kind="stable")
+    degrees = [1008, 1012, 1013, 1016, 1020, 1024]
+    cols = [np.sort(order[:d]) for d in degrees]
+    key = np.unique(np.concatenate([c * len(degrees) + j for j, c in enumerate(cols)]))
+    coo = gb.COOMatrix(rows, len(degrees), (key // len(degrees)).astype(np.int32),
+                       (key % len(degrees)).astype(np.int32))
+    want = np.array([np.sum(np.abs(w[c]) ** 2) for c in cols])
+    got = sums(coo, [0])[0]
+    assert np.all(np.abs(got - want) <= 3e-7 * want)
