@@ -67,7 +67,14 @@ struct gbsp_plan_s {
     int p1_grid = 0;
     size_t p1_smem = 0;
     int rows_grid = 0, rows_threads = 1024, rows_ntmax = 1024;
-    int rows_block = 0;              // launched block (choose_row_block); rows_threads is the planned one
+    // How a launch of n rows runs: the block choose_row_block gives for n
+    // (rows_threads is the planned one) and the CTAs resident at once.  A
+    // single-channel plan holds one entry per block its tiles may get.
+    struct RowsLaunch {
+        gbsp::RowBlock rb;
+        int grid;
+    };
+    std::vector<RowsLaunch> rows_launches;
     int row_mode = 0;                // gbsp::ROW_*
     float2* d_zscratch = nullptr;    // ROW_SEQ: rows_grid x (K-1) x Lp channel results
     size_t rows_smem = 0;
@@ -298,8 +305,13 @@ int launch_pass1(const gbsp_plan_s* p, int u0, int n, float2* S, size_t sp, cons
     return gbsp::p1_launch(p1_kernel(p), p->p1_grid, p->p1_smem, st, pdl, p1_args(p, u0, n, S, sp, chirp));
 }
 
-gbsp::RowsKernel rows_kernel(const gbsp_plan_s* p) {
-    return gbsp::RowsKernel{p->row_mode, p->rows_ntmax, p->K, p->rows_block, p->rows_smem, p->fd.sh < 31};
+gbsp::RowsKernel rows_kernel(const gbsp_plan_s* p, const gbsp::RowBlock& rb) {
+    return gbsp::RowsKernel{p->row_mode, rb.ntmax, p->K, rb.nt, p->rows_smem, p->fd.sh < 31};
+}
+
+gbsp::RowBlock row_block(const gbsp_plan_s* p, int n) {
+    if (p->K != 1) return gbsp::RowBlock{p->rows_threads, p->rows_ntmax};
+    return gbsp::choose_row_block(p->fd, p->rows_threads, n / p->sms, p->direct != 0);
 }
 
 gbsp::RowsArgs rows_args(const gbsp_plan_s* p, const float2* S, size_t s_pitch, int u0, int n, void* d_out,
@@ -329,7 +341,13 @@ gbsp::RowsArgs rows_args(const gbsp_plan_s* p, const float2* S, size_t s_pitch, 
 // the row kernel with fully specified arguments (input tile, output slab
 // and row map)
 int launch_rows_args(const gbsp_plan_s* p, const gbsp::RowsArgs& a, cudaStream_t st, bool pdl = false) {
-    return gbsp::rows_launch(rows_kernel(p), p->rows_grid, st, pdl, a, p->fd, p->d_err);
+    const gbsp::RowBlock rb = row_block(p, a.tile_rows);
+    const gbsp_plan_s::RowsLaunch* l = &p->rows_launches[0];
+    for (const auto& x : p->rows_launches)
+        if (x.rb.nt == rb.nt) l = &x;
+    // no more CTAs (or clusters) than rows
+    const int grid = (int)std::min<long>(l->grid, (long)a.tile_rows * (p->row_mode == gbsp::ROW_CLUSTER ? p->K : 1));
+    return gbsp::rows_launch(rows_kernel(p, l->rb), grid, st, pdl, a, p->fd, p->d_err);
 }
 
 int launch_rows(const gbsp_plan_s* p, int u0, int n, void* d_out, size_t out_pitch, cudaStream_t st,
@@ -338,7 +356,7 @@ int launch_rows(const gbsp_plan_s* p, int u0, int n, void* d_out, size_t out_pit
 }
 
 // Block size and radices are already chosen; pick the compiled variant and
-// size the persistent grid.
+// size the persistent grids.
 int rows_prepare(gbsp_plan_s* p, int sms) {
     int rmax = 0;
     for (int s = 0; s < p->fd.nst; s++) rmax = std::max(rmax, p->fd.R[s]);
@@ -358,17 +376,19 @@ int rows_prepare(gbsp_plan_s* p, int sms) {
         p->fd.sh = 31;
         p->rows_smem = rows_smem_bytes(p->fd);
     }
-    p->rows_block = p->rows_threads;
-    if (p->K == 1) {
-        const RowBlock rb = choose_row_block(p->fd, p->rows_threads, p->u_tile / sms, p->direct != 0);
-        p->rows_block = rb.nt;
-        p->rows_ntmax = rb.ntmax;
+    // a whole tile first, then the wider blocks of smaller ones (streamed
+    // tiles, the last tile)
+    for (int n = p->u_tile;; n /= 2) {
+        const RowBlock rb = row_block(p, n);
+        if (p->rows_launches.empty() || rb.nt != p->rows_launches.back().rb.nt) {
+            int cap = 0;
+            if (int rc = rows_capacity(rows_kernel(p, rb), sms, &cap)) return rc;
+            if (cap < 1) return set_error(GBSP_ERR_UNSUPPORTED, "row kernel does not fit on an SM");
+            p->rows_launches.push_back({rb, (p->row_mode == ROW_CLUSTER) ? cap * p->K : cap});
+        }
+        if (p->K != 1 || n == 0) break;
     }
-    int cap = 0;
-    const int rc = rows_capacity(rows_kernel(p), sms, &cap);
-    if (rc) return rc;
-    if (cap < 1) return set_error(GBSP_ERR_UNSUPPORTED, "row kernel does not fit on an SM");
-    p->rows_grid = (p->row_mode == ROW_CLUSTER) ? cap * p->K : cap;
+    p->rows_grid = p->rows_launches[0].grid;
     return GBSP_OK;
 }
 

@@ -177,7 +177,15 @@ double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct, bo
 // shared memory holds too few rows for that to pay.  At 64 registers a thread
 // more rows fit where shared memory allows (2401 points 380 -> 321 us);
 // radix 16 spills there (2048 points [16, 16, 8] 254 -> 261 us).
+//
+// Few rows fill no SM whatever the block: below 320 threads an SM the block
+// doubles.  Row kernel at 1 to 20 rows an SM and 13 lengths from 70 to 6400
+// points, against the best of the four blocks: 1.0175 on average with the line
+// at 320, 1.086 at 512, 1.026 at 256, 1.045 at 128 (525 points, 7 rows an SM:
+// 16.0, 14.0, 18.1, 27.3 us at 32, 64, 128, 256 threads; 2 rows: 16.0, 10.9,
+// 12.9, 11.9).
 constexpr int BLOCK32_POINTS = 700, BLOCK64_POINTS = 3000, BLOCK128_POINTS = 7000, REGS64_RADIX = 15;
+constexpr int BLOCK_SM_THREADS = 320;
 
 //
 // Long rows (512 threads, one block an SM): a stage of nb butterflies runs
@@ -209,8 +217,8 @@ RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm, bool direc
     }
     if (nt != 256 || fd.Lp > BLOCK128_POINTS) return b;
     b.nt = fd.Lp <= BLOCK32_POINTS ? 32 : fd.Lp <= BLOCK64_POINTS ? 64 : 128;
-    // 512 threads an SM at 128 registers: with fewer rows, wider blocks
-    while (b.nt < nt && rows_per_sm * b.nt < 512) b.nt *= 2;
+    // with too few rows for that, wider blocks
+    while (b.nt < nt && rows_per_sm * b.nt < BLOCK_SM_THREADS) b.nt *= 2;
     if (b.nt <= 64 && rmax <= REGS64_RADIX && (int)(kSmemPerSM / (rows_smem_bytes(fd) + 1024)) > 512 / b.nt)
         b.ntmax = 1024;
     return b;
