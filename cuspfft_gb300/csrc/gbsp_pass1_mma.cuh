@@ -93,6 +93,7 @@ struct P1MmaArgs {
     size_t s_pitch;
     int gtab, tab, ntab, cols, s_cols, rows, u0, tile_rows;
     int nfull, nd_rest;     // row blocks: nfull of MM_MAXD * 128 rows, then one of nd_rest * 128
+    int step_full, step_rest;  // columns per item in these
     uint32_t magic;
     unsigned long long magic64;
     unsigned int* queue;    // [0] next item, [1] CTAs done (zeroed by the last one out)
@@ -103,14 +104,33 @@ struct P1MmaArgs {
 // window (8219 rows: 32 d + 14 rows; two equal blocks would look every A up
 // twice).
 GBSP_HD constexpr int p1_mma_win(int nd) { return nd <= 8 ? 16 : nd <= 16 ? 8 : 4; }
-GBSP_HD inline void p1_mma_tiling(P1MmaArgs* a) {
+GBSP_HD inline int p1_mma_windows(int s_cols, int step) { return (s_cols + step - 1) / step; }
+GBSP_HD inline long p1_mma_items(const P1MmaArgs& a) {
+    return (long)a.nfull * p1_mma_windows(a.s_cols, a.step_full) +
+           (a.nd_rest ? p1_mma_windows(a.s_cols, a.step_rest) : 0);
+}
+// A window's nonzeros are one SM's chain, so with fewer items than SMs (`sms`)
+// a window takes fewer columns than it holds, the widest first: down to four,
+// the epilogue's 32-byte stores, or to one where the chain is longer than the
+// stores (from 32 nonzeros a column, `degree`) or there is an SM for each.
+// GB300, all columns a window holds and fewer: 12001 rows x 64 columns of 200
+// nonzeros 81 -> 25 us, 4097 x 64 of 24 16 -> 14; 8001 x 300 of 100 33 -> 29
+// (of 4, with two columns a window, 16 -> 19).
+GBSP_HD inline void p1_mma_tiling(P1MmaArgs* a, int sms, int degree) {
     const int nd = (a->tile_rows + MM_ROWS - 1) / MM_ROWS;
     a->nfull = nd / MM_BLOCKD;
     a->nd_rest = nd % MM_BLOCKD;
-}
-GBSP_HD inline int p1_mma_windows(int s_cols, int nd) { return (s_cols + p1_mma_win(nd) - 1) / p1_mma_win(nd); }
-GBSP_HD inline long p1_mma_items(const P1MmaArgs& a) {
-    return (long)a.nfull * p1_mma_windows(a.s_cols, MM_BLOCKD) + (a.nd_rest ? p1_mma_windows(a.s_cols, a.nd_rest) : 0);
+    const int least = (degree >= 32 || (a->nfull + 1) * a->s_cols <= sms) ? 1 : 4;
+    a->step_full = a->nfull ? p1_mma_win(MM_BLOCKD) : least;
+    a->step_rest = a->nd_rest ? p1_mma_win(a->nd_rest) : least;
+    for (;;) {
+        P1MmaArgs b = *a;
+        int& step = b.step_rest >= b.step_full ? b.step_rest : b.step_full;
+        if (step <= least) return;
+        step /= 2;
+        if (p1_mma_items(b) > sms) return;
+        *a = b;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -444,7 +464,7 @@ k_twiddle_mma(P1MmaArgs one, const P1MmaArgs* __restrict__ args, const long* __r
         // (3449 rows x 1201 columns, 301 items on 152 SMs: 174 us or 221, by luck).
         struct Next {
             long it;
-            int m, c0, row0, nd, win, k0, kend;
+            int m, c0, row0, nd, step, k0, kend;
             float2 ch;
         } cur;
         int m = 0;
@@ -460,20 +480,21 @@ k_twiddle_mma(P1MmaArgs one, const P1MmaArgs* __restrict__ args, const long* __r
             }
             const P1MmaArgs& a = BATCH ? args[m] : one;
             long i = o.it - first;
-            int n_win = p1_mma_windows(a.s_cols, MM_BLOCKD);
+            int n_win = p1_mma_windows(a.s_cols, a.step_full);
             o.nd = MM_BLOCKD;
+            o.step = a.step_full;
             o.row0 = 0;
             if (i >= (long)a.nfull * n_win) {
                 i -= (long)a.nfull * n_win;
                 o.nd = a.nd_rest;
+                o.step = a.step_rest;
                 o.row0 = a.nfull * MM_BLOCKD * MM_ROWS;
-                n_win = p1_mma_windows(a.s_cols, o.nd);
+                n_win = p1_mma_windows(a.s_cols, o.step);
             }
             const int t = (int)(i / n_win);
             o.row0 += t * MM_BLOCKD * MM_ROWS;
-            o.win = p1_mma_win(o.nd);
-            o.c0 = ((int)i - t * n_win) * o.win;
-            const int j = min(lane, o.win - 1);
+            o.c0 = ((int)i - t * n_win) * o.step;
+            const int j = min(lane, o.step - 1);
             o.k0 = a.kptr[o.c0];
             o.kend = a.kptr[o.c0 + j + 1];
             o.ch = make_float2(MM_UNSCALE, 0.f);
@@ -516,8 +537,8 @@ k_twiddle_mma(P1MmaArgs one, const P1MmaArgs* __restrict__ args, const long* __r
                         q.rows_left = a.tile_rows - cur.row0;
                         q.na = min(MM_ROWS, q.rows_left);
                         q.nd = cur.nd;
-                        q.win = cur.win;
-                        q.ncol = min(cur.win, a.s_cols - cur.c0);
+                        q.win = p1_mma_win(cur.nd);
+                        q.ncol = min(cur.step, a.s_cols - cur.c0);
                         q.used = (int)used;
                         q.vec = (a.s_pitch & 3) == 0 && ((uintptr_t)a.S & 31) == 0;
                     }
@@ -535,7 +556,7 @@ k_twiddle_mma(P1MmaArgs one, const P1MmaArgs* __restrict__ args, const long* __r
                     const int n4 = min(MM_KSTEPS, nk - c * MM_KSTEPS);
                     d.nk = n4;
                     d.kcode = kcode;
-                    d.cstride = MM_TMEM_COLS / cur.win;
+                    d.cstride = MM_TMEM_COLS / p1_mma_win(cur.nd);
                     d.mat = cur.m;
                     d.item = items % MM_ITEMS;
                     d.flags = (c == 0 ? MM_FIRST : 0) | (c == nch - 1 ? MM_LAST : 0);

@@ -260,7 +260,9 @@ gbsp::P1Args p1_args(const gbsp_plan_s* p, int u0, int n, float2* S, size_t s_pi
     return a;
 }
 
-gbsp::P1MmaArgs p1_mma_args(const gbsp_plan_s* p, int u0, int n, float2* S, size_t s_pitch, const float2* chirp) {
+// sms: SMs there are for this matrix
+gbsp::P1MmaArgs p1_mma_args(const gbsp_plan_s* p, int u0, int n, float2* S, size_t s_pitch, const float2* chirp,
+                            int sms) {
     gbsp::P1MmaArgs a;
     a.kfrac = p->d_kfrac;
     a.kptr = p->d_kptr;
@@ -276,7 +278,7 @@ gbsp::P1MmaArgs p1_mma_args(const gbsp_plan_s* p, int u0, int n, float2* S, size
     a.rows = p->rows;
     a.u0 = u0;
     a.tile_rows = n;
-    gbsp::p1_mma_tiling(&a);
+    gbsp::p1_mma_tiling(&a, sms, p->nnz / p->cols);
     a.magic = p->rows_magic;
     a.magic64 = p->rows_magic64;
     a.queue = reinterpret_cast<unsigned int*>(p->d_err + 2);
@@ -301,7 +303,7 @@ constexpr long long MMA_MIN_ROWS_PER_COL = 10000;  // rows x nonzeros per column
 int launch_pass1(const gbsp_plan_s* p, int u0, int n, float2* S, size_t sp, const float2* chirp,
                  cudaStream_t st, bool pdl = false) {
     if (p->mma && n >= MMA_MIN_ROWS)
-        return gbsp::p1_mma_launch(p->sms, p->mma_smem, st, pdl, p1_mma_args(p, u0, n, S, sp, chirp));
+        return gbsp::p1_mma_launch(p->sms, p->mma_smem, st, pdl, p1_mma_args(p, u0, n, S, sp, chirp, p->sms));
     return gbsp::p1_launch(p1_kernel(p), p->p1_grid, p->p1_smem, st, pdl, p1_args(p, u0, n, S, sp, chirp));
 }
 
@@ -1305,10 +1307,11 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
         std::vector<gbsp::P1MmaArgs> mm;
         std::vector<long> p1b(1, 0), mmb(1, 0), rb;
         const int ublk = 32 * b->ku;
+        const int n_mma = (int)std::count_if(b->order.begin(), b->order.end(), [&](int i) { return b->plans[i]->mma; });
         for (int k = 0; k < n; k++) {
             const gbsp_plan_s* p = b->plans[b->order[k]];
             if (p->mma) {
-                mm.push_back(p1_mma_args(p, 0, p->half_rows, p->d_S, p->s_pitch, p1_chirp(p)));
+                mm.push_back(p1_mma_args(p, 0, p->half_rows, p->d_S, p->s_pitch, p1_chirp(p), sms / n_mma));
                 mmb.push_back(mmb.back() + gbsp::p1_mma_items(mm.back()));
                 b->mma_smem = std::max(b->mma_smem, p->mma_smem);
                 continue;

@@ -9,6 +9,10 @@ products, in FP64: the first accumulator loses at most two steps of 2^-14 past
 1024 (1.2e-7 of the sum), the second half a step of its size per MMA, five in
 each of 128 K-steps, 8.4e-5 in all while it grows to 7 (8e-8), and the result
 is rounded once (6e-8): 2.6e-7, held to 3e-7.
+
+Windows.  With few items a window takes fewer columns than it holds.  A sum does
+not depend on its window, so the sums of a narrow matrix are, bit for bit, those
+of the same columns among many.
 """
 import numpy as np
 import pytest
@@ -43,3 +47,28 @@ def test_longest_factors_at_the_degree_limit(cuda, rows):
     want = np.array([np.sum(np.abs(w[c]) ** 2) for c in cols])
     got = sums(coo, [0])[0]
     assert np.all(np.abs(got - want) <= 3e-7 * want)
+
+
+def matrix(rows, degrees, seed):
+    g = np.random.default_rng(seed)
+    r = [g.choice(rows, d, replace=False) for d in degrees]
+    key = np.sort(np.concatenate([x.astype(np.int64) * len(degrees) + j for j, x in enumerate(r)]))
+    return gb.COOMatrix(rows, len(degrees), (key // len(degrees)).astype(np.int32),
+                        (key % len(degrees)).astype(np.int32))
+
+
+# blocks of 32, 16 and fewer d; one and two columns a window and the widest
+@pytest.mark.parametrize("rows", [4097, 4300, 5003, 9001, 12001, 16500])
+@pytest.mark.parametrize("cols", [1, 2, 3, 17, 40, 77, 151, 152, 153, 300])
+@pytest.mark.parametrize("degree", [20, 40])
+def test_sums_do_not_depend_on_the_window(cuda, rows, cols, degree):
+    g = np.random.default_rng(cols)
+    deg = g.integers(max(1, degree - 9), degree + 10, 700)
+    deg[5::7] = 0
+    deg[0] = 60
+    wide = matrix(rows, deg, rows)
+    keep = wide.col_idx < cols
+    narrow = gb.COOMatrix(rows, cols, wide.row_idx[keep].copy(), wide.col_idx[keep].copy())
+    us = np.unique(np.r_[0:300, rows // 4:rows // 4 + 300, rows // 2 - 200:rows // 2 + 1])
+    assert np.array_equal(sums(narrow, us), sums(wide, us)[:, :cols])
+
