@@ -292,12 +292,23 @@ const float2* p1_chirp(const gbsp_plan_s* p) { return p->direct ? nullptr : p->d
 
 // The tensor-core kernel makes the operands of a nonzero at nearly the same
 // cost for any tile of up to 4096 rows, so it needs tall tiles, and enough
-// nonzeros per column to fill its K-steps.  Measured on GB300 (2048 columns,
-// uniform; FP32 time / tensor-core time at 1, 4, 12, 40, 120 nonzeros per
-// column): 1301 rows 0.84 0.97 0.97 1.05 1.15; 2051 rows 0.86 0.91 1.04 1.21
-// 1.38; 2751 rows 0.94 1.04 1.17 1.33 1.57; 6001 rows 1.13 1.25 1.44 1.71 1.92.
+// nonzeros per column to fill its K-steps; with few columns its start (TMEM,
+// table, first chunk), about 3 us longer than the FP32 kernel's, counts too.
+// Rows x nonzeros per column decide, 10000 and for few columns up to 30000.
+// Measured on GB300 (uniform; FP32 time / tensor-core time by nonzeros per
+// column):
+//              columns    1     4     8    12    24   100
+//   2049 rows       64  0.83  0.93  0.94  1.04  1.10  2.08
+//                 1000  0.87  0.94  0.93  1.03  1.05  1.27
+//                 2048  0.84  0.92  1.00  1.03  1.12
+//                 8192  0.93  1.04  1.10  1.19  1.29
+//   2501 rows     1000  0.98  1.01  1.09  1.16  1.30  1.73
+//                 2048  0.90  1.00  1.10  1.18  1.27
+//   4001 rows       64  0.76  0.75  0.82  0.82  1.00  1.67
+//                 2048  0.99  1.09  1.20  1.31  1.47
+//                 8192  1.10  1.26  1.36  1.52  1.74
 constexpr int MMA_MIN_ROWS = 2048;
-constexpr long long MMA_MIN_ROWS_PER_COL = 10000;  // rows x nonzeros per column
+long long mma_min_rows_per_col(int cols) { return 10000 + std::min(20000, 13000000 / cols); }
 
 // chirp == nullptr gives the raw column sums (gbsp_column_sums)
 int launch_pass1(const gbsp_plan_s* p, int u0, int n, float2* S, size_t sp, const float2* chirp,
@@ -445,13 +456,32 @@ int learned_choice(const gbsp_plan_s* p, const int* col_ptr, size_t smem_cap, gb
 // Whether the tensor-core kernel runs pass 1 of a plan's large tiles.  Not in
 // the exact-phase mode (no products of twiddles) nor with an explicit Kahan
 // degree (a property of the FP32 sums), nor with columns past its accumulators'
-// range.
+// range.  Nor where one column's K-steps, which a single CTA runs, would still
+// be running when the others are done (three quarters of all SMs' share; an
+// item's epilogue takes as long as 15 K-steps): the FP32 kernel cuts such a
+// column into parts.  Among columns of similar length (the longest at most six
+// times the mean) its blocks are chains of the same length.  GB300, ten
+// nonzeros a column and one column of more, FP32 time / tensor-core time:
+// 5003 x 2000 250: 1.10, 500: 0.87, 1000: 0.64; 8219^2 1000: 1.08.
 bool mma_choice(const gbsp_plan_s* p, const gbsp_options* o, const int* col_ptr) {
     if (o->exact_phases != 0 || o->kahan_min_degree != 0 || p->mma_tab < 0) return false;
-    if (p->u_tile < MMA_MIN_ROWS || (long long)p->u_tile * p->nnz < MMA_MIN_ROWS_PER_COL * p->cols) return false;
+    if (p->u_tile < MMA_MIN_ROWS ||
+        (long long)p->u_tile * p->nnz < mma_min_rows_per_col(p->cols) * p->cols)
+        return false;
     int most = 0;
-    for (int j = 0; j < p->n_active; j++) most = std::max(most, col_ptr[j + 1] - col_ptr[j]);
-    return most <= gbsp::MM_MAX_DEGREE;
+    long long steps = 0;
+    for (int j = 0; j < p->n_active; j++) {
+        most = std::max(most, col_ptr[j + 1] - col_ptr[j]);
+        steps += (col_ptr[j + 1] - col_ptr[j] + 7) >> 3;
+    }
+    if (most > gbsp::MM_MAX_DEGREE) return false;
+    const long long longest = (most + 7) >> 3;
+    const int nd = (p->u_tile + gbsp::MM_ROWS - 1) / gbsp::MM_ROWS, rest = nd % gbsp::MM_BLOCKD;
+    const long long full = nd / gbsp::MM_BLOCKD;
+    const long long items = full * gbsp::p1_mma_windows(p->cols, gbsp::p1_mma_win(gbsp::MM_BLOCKD)) +
+                            (rest ? gbsp::p1_mma_windows(p->cols, gbsp::p1_mma_win(rest)) : 0);
+    const long long all = steps * (full + (rest ? 1 : 0)) + 15 * items;
+    return longest * p->cols <= 6 * steps || 4 * longest * p->sms <= 3 * all;
 }
 
 // force_p1: 1-based pass-1 shape imposed by a batch (one shape for all its

@@ -58,3 +58,7 @@ def row_launches(fn):
         if "k_bluestein_rows" in name:
             out.append((tuple(int(x) for x in re.findall(r"L[ib](\d+)E", name)), *dims))
     return out
+
+
+def kernel_names(fn):
+    return [name for _, name, _, _ in captured(fn).values() if name]

@@ -13,11 +13,15 @@ is rounded once (6e-8): 2.6e-7, held to 3e-7.
 Windows.  With few items a window takes fewer columns than it holds.  A sum does
 not depend on its window, so the sums of a narrow matrix are, bit for bit, those
 of the same columns among many.
+
+Routes.  Which kernel a matrix gets, read from a captured graph, on both sides of
+each line: rows x nonzeros per column, one column far longer than the others.
 """
 import numpy as np
 import pytest
 
 import cuspfft_gb300 as gb
+from graph_nodes import kernel_names
 
 pytestmark = pytest.mark.gpu
 
@@ -72,3 +76,19 @@ def test_sums_do_not_depend_on_the_window(cuda, rows, cols, degree):
     us = np.unique(np.r_[0:300, rows // 4:rows // 4 + 300, rows // 2 - 200:rows // 2 + 1])
     assert np.array_equal(sums(narrow, us), sums(wide, us)[:, :cols])
 
+
+@pytest.mark.parametrize("rows,degrees,mma", [
+    (4097, [14] * 300, False), (4097, [16] * 300, True),      # 30000 rows x nonzeros a column
+    (4097, [7] * 2048, False), (4097, [9] * 2048, True),      # 16300
+    (8001, [4] * 2048, False), (8001, [5] * 2048, True),
+    (4094, [60] * 300, True), (4093, [60] * 300, False),      # 2048 rows
+    (5003, [10] * 1999 + [250], True), (5003, [10] * 1999 + [1000], False),   # one long column
+    (5003, [1024] * 4, True), (5003, [1024] * 3 + [1025], False)])
+def test_routes(cuda, rows, degrees, mma):
+    import torch
+    coo = matrix(rows, degrees, rows)
+    n = rows // 2 + 1
+    with gb.Plan(coo) as p:
+        s = torch.empty((n, (coo.cols + 1) // 2 * 2), dtype=torch.complex64, device="cuda")
+        [name] = kernel_names(lambda st: p.column_sums(0, n, s, stream=st))
+    assert ("k_twiddle_mma" in name) == mma
