@@ -178,14 +178,18 @@ double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct, bo
 // more rows fit where shared memory allows (2401 points 380 -> 321 us);
 // radix 16 spills there (2048 points [16, 16, 8] 254 -> 261 us).
 //
-// Few rows fill no SM whatever the block: below 320 threads an SM the block
-// doubles.  Row kernel at 1 to 20 rows an SM and 13 lengths from 70 to 6400
-// points, against the best of the four blocks: 1.0175 on average with the line
-// at 320, 1.086 at 512, 1.026 at 256, 1.045 at 128 (525 points, 7 rows an SM:
-// 16.0, 14.0, 18.1, 27.3 us at 32, 64, 128, 256 threads; 2 rows: 16.0, 10.9,
-// 12.9, 11.9).
+// Few rows fill no SM whatever the block, and a narrow one makes the row's own
+// latency longer, most of all where tables and S come from DRAM.  So the block
+// doubles while the SM would have fewer than 256 threads, and 32 threads a row
+// need 18 rows an SM, or 48 from 350 points on.  Whole calls at 1 to 15 rows an
+// SM and ten lengths from 135 to 6400 points, against the best of the four
+// blocks, back to back and by themselves after a write of 256 MB: 1.007 and
+// 1.008 on average (worst 1.07, 1.14); with the line at 512 threads 1.061 and
+// 1.057 (1.33, 1.39), at 320 1.032 and 1.038.  32 and 64 threads, cold, us: 270
+// points 16 rows an SM 42 and 34, 20 40 and 46, 64 103 and 120; 525 points 16
+// 49 and 39, 48 87 and 85, 64 159 and 160.
 constexpr int BLOCK32_POINTS = 700, BLOCK64_POINTS = 3000, BLOCK128_POINTS = 7000, REGS64_RADIX = 15;
-constexpr int BLOCK_SM_THREADS = 320;
+constexpr int BLOCK_SM_THREADS = 256, BLOCK32_SM_ROWS = 18, BLOCK32_LONG_POINTS = 350, BLOCK32_LONG_SM_ROWS = 48;
 
 //
 // Long rows (512 threads, one block an SM): a stage of nb butterflies runs
@@ -218,6 +222,7 @@ RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm, bool direc
     if (nt != 256 || fd.Lp > BLOCK128_POINTS) return b;
     b.nt = fd.Lp <= BLOCK32_POINTS ? 32 : fd.Lp <= BLOCK64_POINTS ? 64 : 128;
     // with too few rows for that, wider blocks
+    if (b.nt == 32 && rows_per_sm < (fd.Lp <= BLOCK32_LONG_POINTS ? BLOCK32_SM_ROWS : BLOCK32_LONG_SM_ROWS)) b.nt = 64;
     while (b.nt < nt && rows_per_sm * b.nt < BLOCK_SM_THREADS) b.nt *= 2;
     if (b.nt <= 64 && rmax <= REGS64_RADIX && (int)(kSmemPerSM / (rows_smem_bytes(fd) + 1024)) > 512 / b.nt)
         b.ntmax = 1024;

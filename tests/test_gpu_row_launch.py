@@ -1,7 +1,7 @@
 """Which block, grid and instance a row launch gets, read from a captured graph.
 
-Short rows run 32, 64 or 128 threads each where that gives every SM 320
-threads, and wider blocks where there are fewer rows; the rows are those of the
+Short rows run 32, 64 or 128 threads each where there are rows enough for
+every SM, and wider blocks where there are fewer; the rows are those of the
 launch, not of the plan.
 """
 import numpy as np
@@ -20,23 +20,23 @@ def sms():
     return torch.cuda.get_device_properties(0).multi_processor_count
 
 
-@pytest.mark.parametrize("full,last", [(16, 16), (16, 9), (16, 5), (16, 1), (8, 7), (8, 3), (4, 1)])
-def test_a_short_tile_gets_a_wider_block(cuda, full, last):
+# rows an SM of the first tile and the second, and their blocks: 525 points (257
+# columns) and 135 (65)
+@pytest.mark.parametrize("cols,full,last,blocks", [
+    (257, 48, 47, (32, 64)), (257, 48, 4, (32, 64)), (257, 16, 3, (64, 128)), (257, 16, 1, (64, 256)),
+    (257, 4, 2, (64, 128)), (257, 2, 1, (128, 256)), (65, 18, 17, (32, 64)), (65, 18, 0, (32, 256))])
+def test_a_short_tile_gets_a_wider_block(cuda, cols, full, last, blocks):
     import torch
     n = sms()
     tile, tail = full * n, last * n + 3
-    rows, cols = 2 * (tile + tail - 1), 257  # tiles of `tile` and `tail` Bluestein rows
+    rows = 2 * (tile + tail - 1)  # tiles of `tile` and `tail` Bluestein rows
     coo = synthetic.uniform_matrix(rows, cols, 4 * rows, seed=rows)
     with gb.Plan(coo, length_policy=gb.GBSP_LEN_7SMOOTH, u_tile=tile) as p:
-        assert p.info["channel_len"] == 525 and p.info["rows_threads"] == 256
+        assert p.info["channel_len"] == {257: 525, 65: 135}[cols] and p.info["rows_threads"] == 256
         out = p.empty_output()
         got = row_launches(lambda st: p.execute(out, stream=st))
-        tails = [tail] if tail <= tile else [tile, tail - tile]
-        assert len(got) == 1 + len(tails)
-        for (_, grid, block), rows_here in zip(got, [tile] + tails):
-            per_sm = rows_here // n
-            assert block == next(b for b in (32, 64, 128, 256) if per_sm * b >= 320 or b == 256)
-            assert grid <= rows_here
+        assert [block for _, _, block in got] == list(blocks)
+        assert got[0][1] <= tile and got[1][1] <= tail
         p.execute(out)
         torch.cuda.synchronize()
         assert p.error_flags() == 0
