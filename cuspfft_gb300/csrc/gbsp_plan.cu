@@ -324,7 +324,7 @@ gbsp::RowsKernel rows_kernel(const gbsp_plan_s* p, const gbsp::RowBlock& rb) {
 
 gbsp::RowBlock row_block(const gbsp_plan_s* p, int n) {
     if (p->K != 1) return gbsp::RowBlock{p->rows_threads, p->rows_ntmax};
-    return gbsp::choose_row_block(p->fd, p->rows_threads, n / p->sms, p->direct != 0);
+    return gbsp::choose_row_block(p->fd, p->rows_threads, (n + p->sms - 1) / p->sms, p->direct != 0);
 }
 
 gbsp::RowsArgs rows_args(const gbsp_plan_s* p, const float2* S, size_t s_pitch, int u0, int n, void* d_out,
@@ -1303,7 +1303,7 @@ int gbsp_batch_create(int count, const gbsp_matrix* mats, const gbsp_options* op
             b->separate.push_back(i);
             continue;
         }
-        rbs[i] = gbsp::choose_row_block(p->fd, p->rows_threads, (int)std::min<long>(all_rows / sms, 1 << 20),
+        rbs[i] = gbsp::choose_row_block(p->fd, p->rows_threads, (int)std::min<long>((all_rows + sms - 1) / sms, 1 << 20),
                                         p->direct != 0);
         rbs[i].ntmax = std::max(rbs[i].ntmax, 512);  // the batched kernel has no 384-thread instance
         if (gbsp::rows_batch_blocks_per_sm(rbs[i], p->fd.sh < 31, rows_smem_bytes(p->fd), &per_sm[i]) != GBSP_OK || per_sm[i] < 1) {

@@ -180,16 +180,15 @@ double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct, bo
 //
 // Few rows fill no SM whatever the block, and a narrow one makes the row's own
 // latency longer, most of all where tables and S come from DRAM.  So the block
-// doubles while the SM would have fewer than 256 threads, and 32 threads a row
-// need 18 rows an SM, or 48 from 350 points on.  Whole calls at 1 to 15 rows an
-// SM and ten lengths from 135 to 6400 points, against the best of the four
-// blocks, back to back and by themselves after a write of 256 MB: 1.007 and
-// 1.008 on average (worst 1.07, 1.14); with the line at 512 threads 1.061 and
-// 1.057 (1.33, 1.39), at 320 1.032 and 1.038.  32 and 64 threads, cold, us: 270
-// points 16 rows an SM 42 and 34, 20 40 and 46, 64 103 and 120; 525 points 16
-// 49 and 39, 48 87 and 85, 64 159 and 160.
+// doubles as long as an SM's rows still run all at once (512 threads at 128
+// registers), and 32 threads a row need 18 rows an SM, or 48 from 350 points on.
+// Whole calls, GB300, us at 64, 128, 256 threads, 1201 columns: 304 rows 21.1
+// at 128 and 17.7 at 256, 608 rows 27.3 at 64 and 22.0 at 128, 730 rows 31, 32
+// and 36, 1186 rows 39, 39 and 49.  32 and 64 threads, after a write of 256 MB:
+// 270 points 16 rows an SM 42 and 34, 20 40 and 46, 64 103 and 120; 525 points
+// 16 49 and 39, 48 87 and 85, 64 159 and 160.
 constexpr int BLOCK32_POINTS = 700, BLOCK64_POINTS = 3000, BLOCK128_POINTS = 7000, REGS64_RADIX = 15;
-constexpr int BLOCK_SM_THREADS = 256, BLOCK32_SM_ROWS = 18, BLOCK32_LONG_POINTS = 350, BLOCK32_LONG_SM_ROWS = 48;
+constexpr int BLOCK_SM_THREADS = 512, BLOCK32_SM_ROWS = 18, BLOCK32_LONG_POINTS = 350, BLOCK32_LONG_SM_ROWS = 48;
 
 //
 // Long rows (512 threads, one block an SM): a stage of nb butterflies runs
@@ -223,7 +222,7 @@ RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm, bool direc
     b.nt = fd.Lp <= BLOCK32_POINTS ? 32 : fd.Lp <= BLOCK64_POINTS ? 64 : 128;
     // with too few rows for that, wider blocks
     if (b.nt == 32 && rows_per_sm < (fd.Lp <= BLOCK32_LONG_POINTS ? BLOCK32_SM_ROWS : BLOCK32_LONG_SM_ROWS)) b.nt = 64;
-    while (b.nt < nt && rows_per_sm * b.nt < BLOCK_SM_THREADS) b.nt *= 2;
+    while (b.nt < nt && (long)rows_per_sm * 2 * b.nt <= BLOCK_SM_THREADS) b.nt *= 2;
     if (b.nt <= 64 && rmax <= REGS64_RADIX && (int)(kSmemPerSM / (rows_smem_bytes(fd) + 1024)) > 512 / b.nt)
         b.ntmax = 1024;
     return b;
@@ -272,7 +271,7 @@ long launch_rows_of(int rows, const gbsp_options* o) {
 }
 
 int split_channels(int cols, long rows, const gbsp_options* o, size_t smem_cap, ChannelSplit* out) {
-    const int rows_per_sm = (int)std::min<long>(rows / kSMs, 1 << 20);
+    const int rows_per_sm = (int)std::min<long>((rows + kSMs - 1) / kSMs, 1 << 20);
     const int policy = (o && o->length_policy) ? o->length_policy : GBSP_LEN_3SMOOTH;
     if (policy != GBSP_LEN_3SMOOTH && policy != GBSP_LEN_7SMOOTH && policy != GBSP_LEN_POW2)
         return set_error(GBSP_ERR_INVALID, "length_policy must be 2, 3 or 7");

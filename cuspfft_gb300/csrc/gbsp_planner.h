@@ -23,7 +23,7 @@ double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct = f
 
 // The block a single-channel row planned for nt threads is launched with, and
 // the compiled block bound of its kernel (384: 168 registers a thread, 512:
-// 128, 1024: 64).  rows_per_sm: rows there are for each SM.
+// 128, 1024: 64).  rows_per_sm: rows an SM gets, rounded up.
 struct RowBlock {
     int nt, ntmax;
 };
