@@ -353,11 +353,41 @@ gbsp::RowsArgs rows_args(const gbsp_plan_s* p, const float2* S, size_t s_pitch, 
 
 // the row kernel with fully specified arguments (input tile, output slab
 // and row map)
-int launch_rows_args(const gbsp_plan_s* p, const gbsp::RowsArgs& a, cudaStream_t st, bool pdl = false) {
-    const gbsp::RowBlock rb = row_block(p, a.tile_rows);
+const gbsp_plan_s::RowsLaunch* rows_launch_of(const gbsp_plan_s* p, int n) {
+    const gbsp::RowBlock rb = row_block(p, n);
     const gbsp_plan_s::RowsLaunch* l = &p->rows_launches[0];
     for (const auto& x : p->rows_launches)
         if (x.rb.nt == rb.nt) l = &x;
+    return l;
+}
+
+// Whether a row launch starts while pass 1 ends (2 to 4 us less).  Its CTAs
+// then land on the SMs that end first, as many as fit; a plain launch spreads
+// them.  So not where one SM would get more rows than the others (the last
+// round of rows, or all of them, on full SMs) and these rows take longer than
+// the start saves: 7500 points, twice that of direct rows, which take half the
+// time.  Not for long launches either, which gain nothing and may lose (16706^2
+// 3132 -> 3305 us), nor for clusters.  Measured on GB300, n rows without / with
+// the early start, back to back, and by themselves after a write of 256 MB (us):
+//   rows alike   608 x 1201 columns  25 / 22, 36 / 32     151 x 8219  40 / 37, 64 / 58
+//   (most - even) * points = 525   151 x 257   15 / 13, 27 / 23
+//                           2401   151 x 1201  18 / 17, 31 / 27
+//                           3150   1520 x 257  25 / 24, 46 / 40
+//                           6400   151 x 3163  27 / 27, 50 / 46;  1001 x 3163  66 / 65, 81 / 77
+//                           9604   1001 x 5003  101 / 112, 119 / 125
+//                          10935   1001 x 601  26 / 33, 36 / 42
+//   clusters     151 x 40421  281 / 384
+constexpr long EARLY_ROWS_POINTS = 32l << 20, EARLY_EXCESS_POINTS = 7500;
+bool rows_start_early(const gbsp_plan_s* p, int n) {
+    if (p->row_mode == gbsp::ROW_CLUSTER || (long)n * p->L > EARLY_ROWS_POINTS) return false;
+    const int grid = rows_launch_of(p, n)->grid;
+    const int per_sm = grid / p->sms, rounds = n / grid, rest = n % grid;
+    const int even = per_sm * rounds + (rest + p->sms - 1) / p->sms, most = per_sm * rounds + std::min(per_sm, rest);
+    return (long)(most - even) * p->L <= EARLY_EXCESS_POINTS * (p->direct ? 2 : 1);
+}
+
+int launch_rows_args(const gbsp_plan_s* p, const gbsp::RowsArgs& a, cudaStream_t st, bool pdl = false) {
+    const gbsp_plan_s::RowsLaunch* l = rows_launch_of(p, a.tile_rows);
     // no more CTAs (or clusters) than rows
     const int grid = (int)std::min<long>(l->grid, (long)a.tile_rows * (p->row_mode == gbsp::ROW_CLUSTER ? p->K : 1));
     return gbsp::rows_launch(rows_kernel(p, l->rb), grid, st, pdl, a, p->fd, p->d_err);
@@ -834,12 +864,6 @@ int check_out(const gbsp_plan_s* p, const void* d_out, size_t out_pitch, const c
 
 }  // namespace
 
-// Row launches of up to this many points start while pass 1 ends (saves ~3 us
-// each: 301 x 257 21.5 -> 15.8 us with both launches); longer ones after it, as
-// they ran slower so (16706^2 3132 -> 3305 us, 8219^2 884 -> 890: pass 1 leaves
-// the SM set for its own shared-memory size).
-static constexpr long PDL_ROWS_POINTS = 32l << 20;
-
 extern "C" {
 
 int gbsp_plan_create(int rows, int cols, int n_active, int nnz, const int* col_ptr,
@@ -925,7 +949,7 @@ int gbsp_execute(gbsp_plan_t p, void* d_out, size_t out_pitch, void* stream) {
     for (int u0 = 0; u0 < p->half_rows; u0 += p->u_tile) {
         const int n = std::min(p->u_tile, p->half_rows - u0);
         if ((rc = launch_pass1(p, u0, n, p->d_S, p->s_pitch, p1_chirp(p), st, true))) return rc;
-        if ((rc = launch_rows(p, u0, n, d_out, out_pitch, st, (long)n * p->L <= PDL_ROWS_POINTS))) return rc;
+        if ((rc = launch_rows(p, u0, n, d_out, out_pitch, st, rows_start_early(p, n)))) return rc;
     }
     return GBSP_OK;
 }

@@ -1,4 +1,4 @@
-"""What a batch's kernels wait for, read from a captured graph.
+"""What kernels wait for, read from captured graphs.
 
 Row kernels read the sums pass 1 wrote, so each needs an edge from every
 pass-1 kernel of its batch; classes of rows run beside one another, so none
@@ -65,3 +65,72 @@ def test_batch_classes_replay_to_the_same_bits(cuda):
                 p.execute(one)
                 torch.cuda.synchronize()
                 assert torch.equal(one, o)
+
+
+def sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+# rows, columns: a small launch, one CTA an SM, rows that fill whole rounds; and
+# rows that would crowd on some SMs, a long launch, clusters
+@pytest.mark.parametrize("n,cols,kw,early", [
+    (151, 257, {}, True), (100, 8219, {}, True), (1000, 8219, {}, True), ("2", 5003, {}, True), ("4", 5003, {}, True),
+    (151, 1201, {}, True), (151, 3163, {}, True), (1001, 5003, {}, False), (1001, 601, {}, False), (76, 11003, {}, False),
+    (4000, 16706, {}, False),
+    (151, 40421, dict(channel_mode=1), False)])
+def test_rows_start_early_only_where_they_spread(cuda, n, cols, kw, early):
+    n = n if isinstance(n, int) else int(n) * sms()
+    coo = synthetic.uniform_matrix(2 * (n - 1), cols, 3 * cols, seed=cols)
+    with gb.Plan(coo, length_policy=gb.GBSP_LEN_7SMOOTH, **kw) as p:
+        assert p.info["half_rows"] == n
+        out = p.empty_output()
+        g = captured(lambda st: p.execute(out, stream=st))
+    [deps] = [d for _, name, d, _ in g.values() if "k_bluestein_rows" in name]
+    assert len(deps) == 1 and "k_twiddle" in g[deps[0][0]][1]
+    assert (deps[0][1] == PROGRAMMATIC) == early
+
+
+def test_execute_is_captured_after_any_node(cuda):
+    # pass 1 carries the attribute of an early start: after a copy, a memset, a join of two streams, a batch
+    import torch
+    coo = synthetic.uniform_matrix(301, 257, 4000, seed=1)
+    mats = [synthetic.uniform_matrix(r, c, 8 * max(r, c), seed=c) for r, c in SHAPES["both"]]
+    with gb.Plan(coo) as p, gb.Batch(mats) as b:
+        want, out, aux = p.empty_output(), p.empty_output(), torch.zeros(1 << 20, device="cuda")
+        bout = b.empty_outputs()
+        b.set_outputs(bout)
+        p.execute(want)
+        torch.cuda.synchronize()
+        side = torch.cuda.Stream()
+
+        def memset(st):
+            aux.zero_()
+
+        def copy(st):
+            aux[: 1 << 19].copy_(aux[1 << 19:])
+
+        def join(st):
+            side.wait_stream(st)
+            with torch.cuda.stream(side):
+                aux.add_(1.0)
+            aux.new_ones(8)
+            st.wait_stream(side)
+
+        def batch(st):
+            b.execute(stream=st)
+
+        for before in (memset, copy, join, batch):
+            graph = torch.cuda.CUDAGraph()
+            out.fill_(complex(np.nan, np.nan))
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph):
+                before(torch.cuda.current_stream())
+                p.execute(out)
+                p.execute(out)
+            for _ in range(2):
+                out.fill_(complex(np.nan, np.nan))
+                graph.replay()
+                torch.cuda.synchronize()
+                assert torch.equal(out, want), before.__name__
+        assert p.error_flags() == 0 and b.error_flags() == 0
