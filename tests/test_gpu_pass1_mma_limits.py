@@ -14,6 +14,12 @@ Windows.  With few items a window takes fewer columns than it holds.  A sum does
 not depend on its window, so the sums of a narrow matrix are, bit for bit, those
 of the same columns among many.
 
+Two-level table.  From some 18000 rows on, and where a half table does not fit
+beside the operands, a factor is a product of two table entries: errors of
+4.3e-8 / sqrt(2) each and the product's 3e-8, four entries and two products a
+term, 5.7e-8 in all when independent; held to 8e-8, and to no more than the FP32
+kernel's on the same sums.
+
 Routes.  Which kernel a matrix gets, read from a captured graph, on both sides of
 each line: rows x nonzeros per column, one column far longer than the others.
 """
@@ -92,3 +98,20 @@ def test_routes(cuda, rows, degrees, mma):
         s = torch.empty((n, (coo.cols + 1) // 2 * 2), dtype=torch.complex64, device="cuda")
         [name] = kernel_names(lambda st: p.column_sums(0, n, s, stream=st))
     assert ("k_twiddle_mma" in name) == mma
+
+
+@pytest.mark.parametrize("rows", [18503, 20001, 30011, 39001, 70001])
+@pytest.mark.parametrize("table", [0, 2, 3])
+def test_two_level_sums_against_fp32(cuda, rows, table):
+    if table == 2 and rows > 39001:
+        pytest.skip("no half table of that many rows")
+    g = np.random.default_rng(rows)
+    coo = matrix(rows, g.integers(2, 300, 48), rows)
+    us = np.unique(np.r_[0:40, rows // 4:rows // 4 + 40, rows // 2 - 40:rows // 2 + 1])
+    ref = np.zeros((us.size, coo.cols), np.complex128)
+    for c in range(coo.cols):
+        r = coo.row_idx[coo.col_idx == c].astype(np.int64)
+        ref[:, c] = np.exp(-2j * np.pi * (np.outer(us, r) % rows) / rows).sum(1)
+    err = [np.linalg.norm(sums(coo, us, row_table_mode=table, **kw) - ref) / np.linalg.norm(ref)
+           for kw in ({}, dict(kahan_min_degree=64))]
+    assert err[0] <= 8e-8 and err[0] <= err[1]

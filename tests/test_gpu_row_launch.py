@@ -2,7 +2,13 @@
 
 Short rows run 32, 64 or 128 threads each where there are rows enough for
 every SM, and wider blocks where there are fewer; the rows are those of the
-launch, not of the plan.
+launch, not of the plan.  Long rows run 352 threads where that divides their
+stages better, two channels that hold the row an instance of their own, and rows
+whose last radix is a power of two a padded buffer.
+
+Spectra are held to rel-L2 1e-6 against FP64, the bar of test_gpu_row_layout.py
+for an FP32 FFT and its inverse of up to five stages; the two or more channels of
+a long row and their sum add one product and one sum each, 1.2e-7.
 """
 import numpy as np
 import pytest
@@ -54,3 +60,43 @@ def test_no_more_blocks_than_rows(cuda):
             out = p.empty_output()
             [(_, grid, _)] = row_launches(lambda st: p.execute(out, stream=st))
             assert grid <= 21 * (p.info["channels"] if kw else 1)
+
+
+SINGLE, SEQ, DIRECT, SEQ2 = 0, 2, 4, 5
+
+
+# rows, columns, options; compiled block bound, kind of row, padded; block (None:
+# as planned, rows of several channels)
+@pytest.mark.parametrize("rows,cols,kw,instance,block", [
+    (401, 8193, dict(length_policy=2), (512, SEQ2, 1), None),
+    (401, 9001, dict(length_policy=2), (512, SEQ2, 1), None),
+    (701, 11003, dict(length_policy=2), (512, SEQ2, 1), None),
+    (401, 16382, dict(length_policy=2), (512, SEQ2, 1), None),
+    (401, 16383, dict(length_policy=2), (512, SEQ2, 1), None),
+    (401, 16706, dict(length_policy=7), (512, SEQ2, 0), None),
+    (401, 16706, dict(length_policy=2), (512, SEQ, 1), None),
+    (401, 40421, dict(length_policy=2), (512, SEQ, 1), None),
+    (401, 40421, dict(length_policy=7), (512, SEQ, 0), None),
+    (401, 8219, dict(length_policy=7), (384, SINGLE, 0), 352),
+    (401, 7499, dict(length_policy=7), (512, SINGLE, 0), 512),
+    (12001, 2048, dict(length_policy=3), (512, DIRECT, 1), 64),
+    (12001, 2401, dict(length_policy=7), (1024, DIRECT, 0), 64),
+    (12001, 1000, dict(length_policy=2), (512, SINGLE, 1), 64),
+    (20001, 257, dict(length_policy=7), (512, SINGLE, 0), 32),
+    (20001, 65, dict(length_policy=7), (1024, SINGLE, 0), 32)])
+def test_instances(cuda, rows, cols, kw, instance, block):
+    import torch
+    coo = synthetic.uniform_matrix(rows, cols, 4 * max(rows, cols), seed=cols)
+    with gb.Plan(coo, **kw) as p:
+        out = p.empty_output()
+        [(args, _, threads)] = row_launches(lambda st: p.execute(out, stream=st))
+        assert (args, threads) == (instance, block or p.info["rows_threads"])
+        out.fill_(complex(7.0, 7.0))
+        p.execute(out)
+        torch.cuda.synchronize()
+        assert p.error_flags() == 0
+        us = np.unique(np.r_[0, 1, rows // 2, rows // 2 + 1, rows - 1, np.arange(5, rows, rows // 12)])
+        got = out[torch.from_numpy(us).cuda()].cpu().numpy()
+    fc = cols // 2 + 1
+    assert np.all(got[:, fc:] == 0)
+    assert fp64.rel_l2(got[:, :fc], fp64.spectrum_rows_fp64(rows, cols, coo.row_idx, coo.col_idx, us)) <= 1e-6
