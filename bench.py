@@ -344,7 +344,7 @@ def run_batched(args, torch, gb, synthetic) -> dict:
                     "density log-uniform in [1e-4, 1e-2], seed 4",
         "unit": "matrices/s", "matrices_per_s": round(64e3 / ms_b, 1), "plain_matrices_per_s": round(64e3 / ms_p, 1),
         "speedup_vs_plain": round(ms_p / ms_b, 3), "ms_per_batch": round(ms_b, 4), "plain_ms_per_batch": round(ms_p, 4),
-        "batched_form": "planner=learned, pass 1 in one work-queue launch, rows in one launch per size class, "
+        "batched_form": "planner=learned, pass 1 in a work-queue launch per kernel, rows in one launch per size class, "
                         "CUDA graph replay; multi-channel matrices through their own plans",
         "plain_form": "64 plans (analytic planner), 2 launches each",
         "multi_channel_matrices": n_sep, "error_flags": flags, "steps": args.batch_steps,

@@ -1,9 +1,10 @@
 // gbsp_launch.h -- host entry points of the kernel translation units.
 //
 // The kernels compile in separate translation units so the build runs them
-// in parallel: pass 1 (gbsp_pass1.cu), single-channel rows and batches
-// (gbsp_rows.cu), multi-channel rows (gbsp_rows_multi.cu).  The plan code
-// (gbsp_plan.cu) reaches them through these functions.
+// in parallel: pass 1 (gbsp_pass1*.cu), single-channel rows (gbsp_rows.cu,
+// _384, _pad), batches of them (gbsp_rows_batch*.cu), multi-channel rows
+// (gbsp_rows_multi.cu, gbsp_rows_seq*.cu).  The plan code (gbsp_plan.cu) reaches
+// them through these functions.
 #pragma once
 #include <cuda_runtime.h>
 

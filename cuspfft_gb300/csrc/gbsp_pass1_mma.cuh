@@ -41,7 +41,10 @@
 //                per column, so a chunk is one bulk copy
 //   warp 21      issues the MMAs, those that share an A part in a row, so that
 //                A stays in the collector buffer
-// Shared-memory bandwidth is what bounds it, so: operands are K-major without
+// No pipe is full (8219^2 on GB300: LSU data pipe 49 %, instruction issue
+// 38 %, tensor pipe 12 %, DRAM the S write alone):
+// a CTA is a chain of operands, MMA and epilogue, and shared memory is its
+// longest link, so: operands are K-major without
 // swizzle (8 x 16-byte core matrices, K halves 2 KB (A) or 1 KB (B) apart), a
 // thread's four nonzeros one 16-byte conflict-free store per part; and table
 // entry p sits at p ^ (p / 16 % 16), because the lookups i*r of consecutive i
@@ -49,7 +52,7 @@
 // The lanes of a warp write 32 consecutive rows of S, a thread's four columns
 // of a row as one 32-byte store (rows 32 apart, one page each, were 2x slower
 // on 40421 columns).  Against the FP32 kernel on GB300: 8219^2 0.34 -> 0.24 ms,
-// 16706^2 1.19 -> 0.69, 40421^2 4.5 -> 2.34, 70001 x 1201 1.21 -> 0.47.
+// 16706^2 1.19 -> 0.68, 40421^2 4.5 -> 2.31, 70001 x 1201 1.21 -> 0.47.
 #pragma once
 #include <cuda_fp16.h>
 #include "gbsp_kernels.cuh"

@@ -1083,15 +1083,16 @@ extern "C" int gbsp_execute_noalloc(gbsp_plan_t p, void* d_out, size_t out_pitch
 }
 
 // ===========================================================================
-// Batches: many matrices of uneven size and sparsity in one persistent
-// launch per pass, fed by device work queues.
+// Batches: many matrices of uneven size and sparsity in a few persistent
+// launches fed by device work queues.
 //
 // Each matrix gets its own tables and scratch (a plan built with a pass-1
 // shape and a block size common to the batch); one descriptor per matrix
-// lists them.  gbsp_batch_execute resets the two queue heads and launches
-// k_twiddle_sum_batch and k_bluestein_rows_batch once each; matrices whose
-// convolution needs several channels run after them through their own plan.
-// The three operations capture into a CUDA graph (gbsp_batch_graph_*).
+// lists them.  gbsp_batch_execute resets the queue heads and launches pass 1
+// (k_twiddle_mma and k_twiddle_sum_batch, whichever matrices there are for) and
+// k_bluestein_rows_batch for each class of rows; matrices whose convolution
+// needs several channels run after them through their own plan.  All of it
+// captures into a CUDA graph (gbsp_batch_graph_*).
 // ===========================================================================
 struct gbsp_batch_s {
     int count = 0;

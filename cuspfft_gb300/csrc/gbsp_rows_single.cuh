@@ -1,6 +1,6 @@
 // gbsp_rows_single.cuh -- launch helpers of the single-channel row kernels,
-// shared by gbsp_rows.cu and gbsp_rows_pad.cu (each compiles its own
-// instances).
+// shared by gbsp_rows.cu, gbsp_rows_384.cu and gbsp_rows_pad.cu (each compiles
+// its own instances).
 #pragma once
 #include "gbsp_launch.h"
 

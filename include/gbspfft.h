@@ -62,13 +62,19 @@ enum { GBSP_PLANNER_MODEL = 0, GBSP_PLANNER_LEARNED = 1 };
  *   2: 256 x 32, half table      3: 128 x 64, full    4: 256 x 16, full
  *   5: 256 x 16, half            6: 128 x 32, half
  *   7: 256 x 32, two-level       8: 128 x 32, two-level (tall matrices)
- * The automatic choice takes the first that fits of 1, 2, 7, 3, 4, 5, 6, 8
- * (measured on GB300); the tuner and the learned planner consider them all.
+ * The automatic choice takes the first that fits of 1, 2, 7, 3, 4, 5, 6, 8,
+ * with tiles (u_tile) of at most 128 rows the first of 3 (from 4096 columns on)
+ * and 6 (measured on GB300); the tuner and the learned planner consider them all.
  * Shapes are those of the FP32 pass 1.  Tiles of at least 2048 Bluestein rows
- * of a matrix with at least 10000 / rows nonzeros per column and none above
- * 1024 run pass 1 on the tensor cores instead, from the same table (sums
- * closer to FP64 than the FP32 ones), unless exact_phases or kahan_min_degree
- * is set. */
+ * run pass 1 on the tensor cores instead where the tile's rows times the mean
+ * nonzeros per column reach 10000 (with few columns up to 30000), no column
+ * has more than 1024 and none so many more than the others that one SM would
+ * outlast the rest, unless exact_phases or kahan_min_degree is set.  These
+ * sums are closer to FP64 than the FP32 ones; their twiddles come from the
+ * shape's table where it fits beside the operands, else from the half table
+ * (the same entries) or the two-level one (products of two).  The two kernels
+ * agree to rounding, so the low bits of a large matrix depend on whether its
+ * tiles have 2048 rows (one launch, u_tile, streaming, the fixed scratch). */
 #define GBSP_N_PASS1_SHAPES 8
 /* Length of the cost-model feature vector (gbsp_plan_features). */
 #define GBSP_N_FEATURES 36
@@ -86,8 +92,9 @@ typedef struct {
     int u_tile;            /* Bluestein rows per tile (each yields output rows u and
                               rows-u); the --csc-tile analogue. 0 = all rows in one tile */
     int kahan_min_degree;  /* columns with >= this many nonzeros accumulate with Kahan
-                              compensation; 0 = default 64; negative = never (plain FP32);
-                              any value but 0 keeps pass 1 on the FP32 kernel       */
+                              compensation; 0 = default: 64 in the FP32 pass 1, none in
+                              the tensor-core one; negative = never (plain FP32); any
+                              value but 0 keeps pass 1 on the FP32 kernel                */
     int index_bytes;       /* 0 = auto (2 when rows,cols <= 65536, else 4), or 2 / 4      */
     int max_channel_len;   /* largest per-CTA FFT length held in shared memory;
                               0 = as long as shared memory allows (about 28k points);
@@ -95,13 +102,16 @@ typedef struct {
                               cluster, or one CTA running them in turn)                   */
     int rows_threads;      /* row-kernel block size: 0 = auto, else a multiple of 32
                               in [64, 1024] (at most 512 when a radix exceeds 16).
-                              Rows of up to 7000 points planned for 256 threads are
-                              launched in blocks of 32, 64 or 128 when there are
-                              enough of them, long ones planned for 512 in 352
-                              where that divides their stages better                      */
+                              A planned size: 256 and 512 name plans (as the tuner and
+                              the learned planner fill them in) whose launches take
+                              blocks of 32, 64 or 128 for rows of up to 7000 points when
+                              there are enough of them, and of 352 for long ones where
+                              that divides their stages better.  Any other number is
+                              launched as it is                                           */
     int row_table_mode;    /* pass-1 twiddle table: 0 = auto, 1 = full circle,
                               2 = half circle, 3 = two-level (W^p = hi[p/256]*lo[p%256],
-                              any row count)                                              */
+                              any row count); the tensor-core pass 1 takes a coarser one
+                              where this one does not fit beside its operands             */
     int radix[8];          /* channel FFT radix per stage, first to last, 0-terminated;
                               all zero = auto.  Allowed: 2 3 4 5 7 8 9 12 15 16 20 21
                               24 25 28 32 35 40; product = channel length                 */
@@ -140,8 +150,8 @@ typedef struct {
     int half_rows;         /* rows/2 + 1 Bluestein rows (Hermitian pairing)              */
     int u_tile;            /* effective Bluestein rows per tile                           */
     int index_bytes;       /* 2 or 4                                                      */
-    int row_table_mode;    /* pass-1 table in shared memory: 0 full, 1 half, 2 two-level  */
-    int rows_threads;      /* row-kernel block size in use                                */
+    int row_table_mode;    /* table of the pass-1 shape: 0 full, 1 half, 2 two-level      */
+    int rows_threads;      /* planned row-kernel block size (see gbsp_options)            */
     size_t device_bytes;   /* device memory held by the plan                              */
     int pass1_shape;       /* pass-1 shape in use (1-based)                               */
     int planner;           /* planner that chose the configuration (GBSP_PLANNER_MODEL
@@ -235,10 +245,11 @@ int gbsp_column_sums(gbsp_plan_t plan, int u0, int n_rows, void* d_s, size_t s_p
  * counterpart in the reference).  For callers that must not allocate device
  * memory while they run transforms -- device memory owned by a pool with a
  * hard budget, or latency-critical code that cannot afford cudaMalloc's
- * implicit synchronisation: it computes the same result as gbsp_execute, but
- * the pass-1 intermediate lives in a fixed 32 MiB array inside the library
- * (held by every GPU that loads the library until the process exits) and no
- * allocating routine is called.
+ * implicit synchronisation: it computes the same result as gbsp_execute (to
+ * rounding where that runs pass 1 on the tensor cores and these tiles are too
+ * small for it), but the pass-1 intermediate lives in a fixed 32 MiB array
+ * inside the library (held by every GPU that loads the library until the
+ * process exits) and no allocating routine is called.
  *   - The plan's device must be current.  The first call on each device looks
  *     up the array's device address and keeps it; make that first call before
  *     any stream capture.  The address belongs to the device's context:
@@ -299,9 +310,10 @@ int gbsp_device_flags_status(int flags);
  * gbsp_batch_create builds one sub-plan per matrix (same tables as
  * gbsp_plan_create, with one pass-1 shape common to the batch; opts'
  * u_tile, rows_threads and radix are ignored: each matrix gets the
- * planner's automatic radices and row block).  Pass 1 of all matrices is one
- * launch; the Bluestein rows are one launch per class of matrices sharing a
- * block size and CTAs-per-SM count.  Matrices whose convolution needs
+ * planner's automatic radices and row block).  Pass 1 is one launch, or one per
+ * kernel where some matrices take the tensor cores; the Bluestein rows are one
+ * launch per class of matrices sharing a block size and CTAs-per-SM count, on
+ * streams of the batch's own that wait for `stream` and that it waits for.  Matrices whose convolution needs
  * several channels (thread-block clusters) run after the batched launches
  * through their own sub-plan.  Outputs are bound once with
  * gbsp_batch_set_outputs (same rules as gbsp_execute's d_out / out_pitch);
