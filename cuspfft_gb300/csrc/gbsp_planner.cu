@@ -228,6 +228,16 @@ RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm, bool direc
     return b;
 }
 
+// The block the ranking weighs the radices of a short row at (the weights of
+// rows_cost were fitted so): 512 threads an SM.  Of its own, so that the radices
+// of a matrix, and with them its bits, do not follow the block of a launch.
+static int ranking_block(const FFTDesc& fd, int rows_per_sm) {
+    if (fd.Lp > BLOCK128_POINTS) return 256;
+    int nt = fd.Lp <= BLOCK32_POINTS ? 32 : fd.Lp <= BLOCK64_POINTS ? 64 : 128;
+    while (nt < 256 && rows_per_sm * nt < 512) nt *= 2;
+    return nt;
+}
+
 std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_opt, int nt_opt, bool direct,
                                     bool single, int rows_per_sm) {
     std::vector<std::vector<int>> cands;
@@ -255,8 +265,7 @@ std::vector<RadixPlan> rank_radices(int Lp, size_t smem_cap, const int* radix_op
             RadixPlan rp;
             rp.fd = fd;
             rp.nt = nt;
-            // at the block it is launched with
-            const int block = single && nt == 256 ? choose_row_block(fd, nt, rows_per_sm, direct).nt : nt;
+            const int block = single && nt == 256 ? ranking_block(fd, rows_per_sm) : nt;
             rp.cost = rows_cost(fd, block, rows_smem_bytes(fd), direct);
             out.push_back(rp);
         }
@@ -271,7 +280,7 @@ long launch_rows_of(int rows, const gbsp_options* o) {
 }
 
 int split_channels(int cols, long rows, const gbsp_options* o, size_t smem_cap, ChannelSplit* out) {
-    const int rows_per_sm = (int)std::min<long>((rows + kSMs - 1) / kSMs, 1 << 20);
+    const int rows_per_sm = (int)std::min<long>(rows / kSMs, 1 << 20);
     const int policy = (o && o->length_policy) ? o->length_policy : GBSP_LEN_3SMOOTH;
     if (policy != GBSP_LEN_3SMOOTH && policy != GBSP_LEN_7SMOOTH && policy != GBSP_LEN_POW2)
         return set_error(GBSP_ERR_INVALID, "length_policy must be 2, 3 or 7");
