@@ -292,11 +292,13 @@ const float2* p1_chirp(const gbsp_plan_s* p) { return p->direct ? nullptr : p->d
 
 // The tensor-core kernel makes the operands of a nonzero at nearly the same
 // cost for any tile of up to 4096 rows, so it needs tall tiles, and enough
-// nonzeros per column to fill its K-steps; with few columns its start (TMEM,
-// table, first chunk), about 3 us longer than the FP32 kernel's, counts too.
-// Rows x nonzeros per column decide, 10000 and for few columns up to 30000.
-// Measured on GB300 (uniform; FP32 time / tensor-core time by nonzeros per
-// column):
+// nonzeros per column to fill its K-steps.  From 10000 rows x nonzeros per
+// column on it is as fast as the FP32 kernel or within some 7 % (with few
+// columns, where its start -- TMEM, table, first chunk -- is 2 us longer, some
+// 15 %), and its sums are three times closer to FP64 (3e-8 against 1e-7; 4907 x
+// 763 with 4 nonzeros a column: the spectrum 1.85e-7 against 2.00e-7), which
+// decides there.  Measured on GB300 (uniform; FP32 time / tensor-core time by
+// nonzeros per column):
 //              columns    1     4     8    12    24   100
 //   2049 rows       64  0.83  0.93  0.94  1.04  1.10  2.08
 //                 1000  0.87  0.94  0.93  1.03  1.05  1.27
@@ -308,7 +310,7 @@ const float2* p1_chirp(const gbsp_plan_s* p) { return p->direct ? nullptr : p->d
 //                 2048  0.99  1.09  1.20  1.31  1.47
 //                 8192  1.10  1.26  1.36  1.52  1.74
 constexpr int MMA_MIN_ROWS = 2048;
-long long mma_min_rows_per_col(int cols) { return 10000 + std::min(20000, 13000000 / cols); }
+constexpr long long MMA_MIN_ROWS_PER_COL = 10000;  // rows x nonzeros per column
 
 // chirp == nullptr gives the raw column sums (gbsp_column_sums)
 int launch_pass1(const gbsp_plan_s* p, int u0, int n, float2* S, size_t sp, const float2* chirp,
@@ -495,9 +497,7 @@ int learned_choice(const gbsp_plan_s* p, const int* col_ptr, size_t smem_cap, gb
 // 5003 x 2000 250: 1.10, 500: 0.87, 1000: 0.64; 8219^2 1000: 1.08.
 bool mma_choice(const gbsp_plan_s* p, const gbsp_options* o, const int* col_ptr) {
     if (o->exact_phases != 0 || o->kahan_min_degree != 0 || p->mma_tab < 0) return false;
-    if (p->u_tile < MMA_MIN_ROWS ||
-        (long long)p->u_tile * p->nnz < mma_min_rows_per_col(p->cols) * p->cols)
-        return false;
+    if (p->u_tile < MMA_MIN_ROWS || (long long)p->u_tile * p->nnz < MMA_MIN_ROWS_PER_COL * p->cols) return false;
     int most = 0;
     long long steps = 0;
     for (int j = 0; j < p->n_active; j++) {

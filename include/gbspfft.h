@@ -67,9 +67,9 @@ enum { GBSP_PLANNER_MODEL = 0, GBSP_PLANNER_LEARNED = 1 };
  * and 6 (measured on GB300); the tuner and the learned planner consider them all.
  * Shapes are those of the FP32 pass 1.  Tiles of at least 2048 Bluestein rows
  * run pass 1 on the tensor cores instead where the tile's rows times the mean
- * nonzeros per column reach 10000 (with few columns up to 30000), no column
- * has more than 1024 and none so many more than the others that one SM would
- * outlast the rest, unless exact_phases or kahan_min_degree is set.  These
+ * nonzeros per column reach 10000, no column has more than 1024 and none so
+ * many more than the others that one SM would outlast the rest, unless
+ * exact_phases or kahan_min_degree is set.  These
  * sums are closer to FP64 than the FP32 ones; their twiddles come from the
  * shape's table where it fits beside the operands, else from the half table
  * (the same entries) or the two-level one (products of two).  The two kernels

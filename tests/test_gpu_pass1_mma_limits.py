@@ -84,9 +84,9 @@ def test_sums_do_not_depend_on_the_window(cuda, rows, cols, degree):
 
 
 @pytest.mark.parametrize("rows,degrees,mma", [
-    (4097, [14] * 300, False), (4097, [16] * 300, True),      # 30000 rows x nonzeros a column
-    (4097, [7] * 2048, False), (4097, [9] * 2048, True),      # 16300
-    (8001, [4] * 2048, False), (8001, [5] * 2048, True),
+    (4097, [4] * 300, False), (4097, [5] * 300, True),        # 10000 rows x nonzeros a column
+    (4097, [4] * 2048, False), (4097, [5] * 2048, True),
+    (8001, [2] * 2048, False), (8001, [3] * 2048, True),
     (4094, [60] * 300, True), (4093, [60] * 300, False),      # 2048 rows
     (5003, [10] * 1999 + [250], True), (5003, [10] * 1999 + [1000], False),   # one long column
     (5003, [1024] * 4, True), (5003, [1024] * 3 + [1025], False)])
