@@ -181,14 +181,15 @@ double rows_cost(const FFTDesc& fd, int nt, size_t smem_per_cta, bool direct, bo
 // Few rows fill no SM whatever the block, and a narrow one makes the row's own
 // latency longer, most of all where tables and S come from DRAM.  So the block
 // doubles as long as an SM's rows still run all at once (512 threads at 128
-// registers), and 32 threads a row need 18 rows an SM, or 48 from 350 points on.
-// Whole calls, GB300, us at 64, 128, 256 threads, 1201 columns: 304 rows 21.1
-// at 128 and 17.7 at 256, 608 rows 27.3 at 64 and 22.0 at 128, 730 rows 31, 32
-// and 36, 1186 rows 39, 39 and 49.  32 and 64 threads, after a write of 256 MB:
-// 270 points 16 rows an SM 42 and 34, 20 40 and 46, 64 103 and 120; 525 points
-// 16 49 and 39, 48 87 and 85, 64 159 and 160.
+// registers), and 32 threads a row need 18 rows an SM.  Whole calls at 1 to 64
+// rows an SM and 11 lengths from 135 to 6400 points, against the best of the
+// four blocks, back to back and by themselves after a write of 256 MB: 1.017
+// and 1.010 on average (worst 1.17, 1.13).  GB300, us at 64, 128, 256 threads,
+// 1201 columns: 304 rows 23.8, 21.8, 17.8; 608 rows 27.3, 22.1, 27.2; 760 rows
+// 31.0, 35.0, 36.2.  32 and 64 threads, 257 columns: 16 rows an SM 31.6 and
+// 29.3, cold 45.7 and 39.5; 20 rows 41.5 and 48.3, 62.1 and 68.2.
 constexpr int BLOCK32_POINTS = 700, BLOCK64_POINTS = 3000, BLOCK128_POINTS = 7000, REGS64_RADIX = 15;
-constexpr int BLOCK_SM_THREADS = 512, BLOCK32_SM_ROWS = 18, BLOCK32_LONG_POINTS = 350, BLOCK32_LONG_SM_ROWS = 48;
+constexpr int BLOCK_SM_THREADS = 512, BLOCK32_SM_ROWS = 18;
 
 //
 // Long rows (512 threads, one block an SM): a stage of nb butterflies runs
@@ -221,7 +222,7 @@ RowBlock choose_row_block(const FFTDesc& fd, int nt, int rows_per_sm, bool direc
     if (nt != 256 || fd.Lp > BLOCK128_POINTS) return b;
     b.nt = fd.Lp <= BLOCK32_POINTS ? 32 : fd.Lp <= BLOCK64_POINTS ? 64 : 128;
     // with too few rows for that, wider blocks
-    if (b.nt == 32 && rows_per_sm < (fd.Lp <= BLOCK32_LONG_POINTS ? BLOCK32_SM_ROWS : BLOCK32_LONG_SM_ROWS)) b.nt = 64;
+    if (b.nt == 32 && rows_per_sm < BLOCK32_SM_ROWS) b.nt = 64;
     while (b.nt < nt && (long)rows_per_sm * 2 * b.nt <= BLOCK_SM_THREADS) b.nt *= 2;
     if (b.nt <= 64 && rmax <= REGS64_RADIX && (int)(kSmemPerSM / (rows_smem_bytes(fd) + 1024)) > 512 / b.nt)
         b.ntmax = 1024;

@@ -29,7 +29,7 @@ def sms():
 # rows an SM of the first tile (all alike) and the second (one SM has another
 # row), and their blocks: 525 points (257 columns) and 135 (65)
 @pytest.mark.parametrize("cols,full,last,blocks", [
-    (257, 48, 46, (32, 64)), (257, 48, 4, (32, 64)), (257, 16, 3, (64, 128)), (257, 16, 1, (64, 256)),
+    (257, 18, 16, (32, 64)), (257, 18, 4, (32, 64)), (257, 16, 3, (64, 128)), (257, 16, 1, (64, 256)),
     (257, 8, 7, (64, 64)), (257, 4, 2, (128, 128)), (257, 2, 1, (256, 256)), (65, 18, 16, (32, 64)),
     (65, 18, 0, (32, 256))])
 def test_a_short_tile_gets_a_wider_block(cuda, cols, full, last, blocks):
